@@ -3,10 +3,10 @@ optional per-group affine, as torch tensors ready for HelixLinear.
 
 Follows the reference writer's algorithm (helix_substrate/hxq_writer_v3.py:162-232,
 422-467; k-means helix_substrate/hxq_encoder.py:107-207; outliers
-helix_substrate/generate_sidecars_v3.py:18-40) but runs on the GPU with plain
-torch ops, because CPU k-means takes about a minute per 16 M-element tensor and
-a 7B model has 196 of them.  It is the caller feeding the forward path, not part
-of the timed path.
+helix_substrate/generate_sidecars_v3.py:18-40) but runs on the GPU, because CPU
+k-means takes about a minute per 16 M-element tensor and a 7B model has 196 of
+them.  On a CUDA device the passes over the weight are kernels (csrc/hxq_encode.cu);
+a CPU tensor takes the same steps in plain torch ops.
 
 Nearest-centroid assignment uses the sorted codebook's midpoints
 (``bucketize``): for a strictly increasing codebook this gives the same index as
@@ -16,14 +16,33 @@ data), where the reference takes the lower index and so does ``right=False``.
 
 from __future__ import annotations
 
+import ctypes as C
+import math
 from typing import Optional
 
 import torch
+
+from . import _lib
 
 _KMEANS_MAX_SAMPLES = 500_000
 
 
 _subsample_cache: dict = {}
+_subsample_on_device: dict = {}     # (n, device) -> the same positions, for the sizes in use: at most _SUBSAMPLE_KEEP
+_SUBSAMPLE_KEEP = 8                 # tables of 4 MB
+
+
+def _ptr(t: torch.Tensor) -> C.c_void_p:
+    return C.c_void_p(t.data_ptr())
+
+
+def _stream(device: torch.device) -> C.c_void_p:
+    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def _f32_on_gpu(t: torch.Tensor) -> bool:
+    """Values the kernels can take without rounding them: fp32, or 16-bit floats widened to it."""
+    return t.is_cuda and t.dtype in (torch.float32, torch.float16, torch.bfloat16) and t.numel() > 0
 
 
 def _subsample_positions(n: int) -> torch.Tensor:
@@ -39,6 +58,31 @@ def _subsample_positions(n: int) -> torch.Tensor:
     return pos
 
 
+def _subsample_positions_on(n: int, device: torch.device) -> torch.Tensor:
+    """``_subsample_positions`` on a device, kept for the few sizes a model's tensors have: the copy
+    of 500 000 positions from pageable memory took longer than the k-means it feeds."""
+    key = (n, device.index if device.index is not None else torch.cuda.current_device())
+    pos = _subsample_on_device.get(key)
+    if pos is None:
+        pos = _subsample_positions(n).to(device)          # complete on return: a copy from pageable memory
+        while len(_subsample_on_device) >= _SUBSAMPLE_KEEP:
+            _subsample_on_device.pop(next(iter(_subsample_on_device)), None)
+        _subsample_on_device[key] = pos
+    pos.record_stream(torch.cuda.current_stream(device))  # a table that is dropped outlives its use on this stream
+    return pos
+
+
+def _kmeans_on_gpu(sample: torch.Tensor, n_clusters: int, max_iters: int, rtol: float) -> torch.Tensor:
+    """Lloyd on a sorted fp32 sample: runs between midpoints, sums as differences of fp64 prefix sums."""
+    prefix = torch.where(sample.isfinite(), sample.double(), 0.0).cumsum(0)
+    cents = torch.empty(n_clusters, dtype=torch.float32, device=sample.device)
+    with torch.cuda.device(sample.device):
+        st = _lib.lib().hxq_encode_kmeans(_ptr(sample), _ptr(prefix), sample.numel(), n_clusters, max_iters, rtol,
+                                          _ptr(cents), _stream(sample.device))
+    _lib.check(st, "hxq_encode_kmeans")
+    return cents
+
+
 def kmeans_codebook(flat: torch.Tensor, n_clusters: int = 256, max_iters: int = 10,
                     rtol: float = 1e-3) -> torch.Tensor:
     """1-D Lloyd on the reference's RandomState(42) subsample with percentile
@@ -48,10 +92,12 @@ def kmeans_codebook(flat: torch.Tensor, n_clusters: int = 256, max_iters: int = 
     reference writer makes - indices are always the nearest entry of whichever codebook is given."""
     n = flat.numel()
     if n > _KMEANS_MAX_SAMPLES:
-        sample = flat[_subsample_positions(n).to(flat.device)]
+        sample = flat[_subsample_positions_on(n, flat.device) if flat.is_cuda else _subsample_positions(n).to(flat.device)]
     else:
         sample = flat
     sample = sample.float().sort().values
+    if flat.is_cuda and flat.ndim == 1 and n > 0 and 1 <= n_clusters <= 256:
+        return _kmeans_on_gpu(sample, n_clusters, max_iters, rtol)
     q = torch.linspace(0, 1, n_clusters, device=flat.device, dtype=torch.float64)
     pos = q * (sample.numel() - 1)
     lo = pos.floor().long()
@@ -73,6 +119,13 @@ def kmeans_codebook(flat: torch.Tensor, n_clusters: int = 256, max_iters: int = 
 
 def assign_indices(flat: torch.Tensor, codebook: torch.Tensor) -> torch.Tensor:
     """Nearest entry of a sorted codebook, uint8."""
+    if _f32_on_gpu(flat) and _f32_on_gpu(codebook) and codebook.device == flat.device and codebook.ndim == 1 and codebook.numel() <= 256:
+        src, cb32 = flat.float().contiguous(), codebook.float().contiguous()
+        out = torch.empty(flat.shape, dtype=torch.uint8, device=flat.device)
+        with torch.cuda.device(flat.device):
+            st = _lib.lib().hxq_encode_assign(_ptr(src), src.numel(), _ptr(cb32), cb32.numel(), _ptr(out), _stream(flat.device))
+        _lib.check(st, "hxq_encode_assign")
+        return out
     cb = codebook.double()
     mids = ((cb[1:] + cb[:-1]) * 0.5).contiguous()     # exact in fp64: a rounded fp32 midpoint misplaces values next to it
     out = torch.empty(flat.numel(), dtype=torch.uint8, device=flat.device)
@@ -83,19 +136,57 @@ def assign_indices(flat: torch.Tensor, codebook: torch.Tensor) -> torch.Tensor:
     return out.view(flat.shape)
 
 
+def _outliers_on_gpu(flat: torch.Tensor, rank_lo: int, rank_hi: int):
+    """Values beyond the order statistics of two (0-based) ranks: two selections in three passes, a count per
+    run of values, and the positions."""
+    L, n, dev = _lib.lib(), flat.numel(), flat.device
+    thr = torch.empty(2, dtype=torch.float32, device=dev)
+    ws = torch.empty(L.hxq_encode_select_workspace_bytes(), dtype=torch.uint8, device=dev)
+    counts = torch.empty(L.hxq_encode_outlier_runs(n), dtype=torch.int32, device=dev)
+    with torch.cuda.device(dev):
+        s = _stream(dev)
+        _lib.check(L.hxq_encode_select2(_ptr(flat), n, rank_lo, rank_hi, _ptr(thr), _ptr(ws), ws.numel(), s), "hxq_encode_select2")
+        _lib.check(L.hxq_encode_outliers(_ptr(flat), n, _ptr(thr), _ptr(counts), None, None, None, s), "hxq_encode_outliers")
+        ends = counts.cumsum(0)
+        total = int(ends[-1])
+        pos = torch.empty(total, dtype=torch.int64, device=dev)
+        vals = torch.empty(total, dtype=torch.float32, device=dev)
+        if total:
+            _lib.check(L.hxq_encode_outliers(_ptr(flat), n, _ptr(thr), None, _ptr(ends), _ptr(pos), _ptr(vals), s), "hxq_encode_outliers")
+    return pos, vals
+
+
 def find_outliers_percentile(weight: torch.Tensor, percentile: float):
     """Two-sided percentile outliers: positions ascending, fp32 values."""
     flat = weight.reshape(-1).float()
     n = flat.numel()
     # numpy's linear-interpolated percentile lies between two order statistics;
     # "beyond it" is therefore decided by the order statistic on its inner side.
-    import math
     pos_hi = (n - 1) * (percentile / 100.0)
     pos_lo = (n - 1) * ((100.0 - percentile) / 100.0)
+    if flat.is_cuda and 0 < n <= 0xffffffff:
+        return _outliers_on_gpu(flat.contiguous(), min(n, int(math.ceil(pos_lo)) + 1) - 1, min(n, int(math.floor(pos_hi)) + 1) - 1)
     hi = torch.kthvalue(flat, min(n, int(math.floor(pos_hi)) + 1)).values
     lo = torch.kthvalue(flat, min(n, int(math.ceil(pos_lo)) + 1)).values
     pos = torch.nonzero((flat < lo) | (flat > hi)).reshape(-1)
     return pos, flat[pos]
+
+
+def _fit_on_gpu(weight: torch.Tensor, codebook: torch.Tensor, indices: torch.Tensor, group_size: int,
+                exclude: Optional[torch.Tensor], ascending: bool = False):
+    n_out, n_in = weight.shape
+    w, cb, idx = weight.float().contiguous(), codebook.float(), indices.contiguous()
+    cb = torch.cat([cb, cb[-1:].expand(256 - cb.numel())]) if cb.numel() < 256 else cb.contiguous()
+    n_ex = 0 if exclude is None else exclude.numel()
+    if n_ex and not ascending:
+        exclude = torch.where(exclude < 0, exclude + w.numel(), exclude).sort().values
+    s = torch.empty(n_out, n_in // group_size, dtype=torch.float32, device=w.device)
+    t = torch.empty_like(s)
+    with torch.cuda.device(w.device):
+        st = _lib.lib().hxq_encode_fit(_ptr(w), _ptr(idx), _ptr(cb), s.numel(), group_size, _ptr(exclude) if n_ex else None, n_ex,
+                                       _ptr(s), _ptr(t), _stream(w.device))
+    _lib.check(st, "hxq_encode_fit")
+    return s, t
 
 
 def fit_group_affine(weight: torch.Tensor, codebook: torch.Tensor, indices: torch.Tensor,
@@ -104,6 +195,11 @@ def fit_group_affine(weight: torch.Tensor, codebook: torch.Tensor, indices: torc
     positions left out of the fit.  fp64 sums, fp32 result."""
     n_out, n_in = weight.shape
     ng = n_in // group_size
+    if (_f32_on_gpu(weight) and _f32_on_gpu(codebook) and codebook.ndim == 1 and codebook.numel() <= 256 and ng * group_size == n_in
+            and indices.shape == weight.shape and indices.dtype == torch.uint8
+            and codebook.device == weight.device and indices.device == weight.device
+            and (exclude is None or (exclude.dtype == torch.int64 and exclude.ndim == 1 and exclude.device == weight.device))):
+        return _fit_on_gpu(weight, codebook, indices, group_size, exclude)
     w = weight.double().view(n_out, ng, group_size)
     c = codebook.double()[indices.long()].view(n_out, ng, group_size)
     m = torch.ones(n_out * n_in, dtype=torch.float64, device=weight.device)
@@ -147,7 +243,8 @@ def compress_weight(weight: torch.Tensor, n_clusters: int = 256, percentile: flo
         out["sidecar_values"] = vals.half().float()
     if group_size > 0:
         assert w.shape[1] % group_size == 0
-        s, t = fit_group_affine(w, cb, idx, group_size, pos)
+        # (the sidecar's positions ascend already)
+        s, t = _fit_on_gpu(w, cb, idx, group_size, pos, ascending=True) if w.is_cuda and w.numel() else fit_group_affine(w, cb, idx, group_size, pos)
         out["group_scales"], out["group_offsets"] = s.to(st_dtype), t.to(st_dtype)
         out["group_size"] = group_size
     return out

@@ -275,6 +275,35 @@ int hxq_allreduce_add_rmsnorm(void* const* peer_buffers, void* const* peer_flags
                               int64_t wait_cycles, int32_t* status, hxq_stream_t stream);
 
 /*
+ * ---- the encoder's passes over a dense fp32 weight (all pointers DEVICE pointers) ----
+ * What the reference writer does on the host with numpy (helix_substrate/hxq_encoder.py:107-207,
+ * hxq_writer_v3.py:162-232, generate_sidecars_v3.py:18-40), one streaming pass each.
+ */
+/* out[0], out[1]: the values of 0-based ranks rank0 and rank1 of v[0..n) in ascending order, NaNs last
+ * (n < 2^32).  workspace: hxq_encode_select_workspace_bytes() of 8-byte aligned scratch. */
+size_t hxq_encode_select_workspace_bytes(void);
+int hxq_encode_select2(const float* v, int64_t n, int64_t rank0, int64_t rank1, float* out, void* workspace,
+                       size_t workspace_bytes, hxq_stream_t stream);
+/* k <= 256 centroids of an ascending sample: percentile start, at most max_iters Lloyd steps, stop before the
+ * first step that moves no centroid by rtol of the start's range.  prefix: inclusive fp64 prefix sums of the
+ * sample with its non-finite values counted as zero. */
+int hxq_encode_kmeans(const float* sorted, const double* prefix, int32_t n, int32_t k, int32_t max_iters,
+                      double rtol, float* centroids, hxq_stream_t stream);
+/* indices[i] = number of midpoints of the ascending codebook (k <= 256) that lie below w[i]: the nearest entry,
+ * the lower one at a tie. */
+int hxq_encode_assign(const float* w, int64_t n, const float* codebook, int32_t k, uint8_t* indices, hxq_stream_t stream);
+/* Values below thresholds[0] or above thresholds[1].  With counts: their number in each of the
+ * hxq_encode_outlier_runs(n) runs.  With counts == NULL: positions (ascending) and values, ends being the
+ * inclusive prefix sums of the counts. */
+int64_t hxq_encode_outlier_runs(int64_t n);
+int hxq_encode_outliers(const float* w, int64_t n, const float* thresholds, int32_t* counts, const int64_t* ends,
+                        int64_t* positions, float* values, hxq_stream_t stream);
+/* Least squares of w on codebook[indices] (256 entries) per run of group_size values, the n_exclude ascending
+ * flat positions left out; fp64 sums, fp32 results. */
+int hxq_encode_fit(const float* w, const uint8_t* indices, const float* codebook, int64_t n_groups, int32_t group_size,
+                   const int64_t* exclude, int64_t n_exclude, float* scales, float* offsets, hxq_stream_t stream);
+
+/*
  * Host helper: CSR row pointer from ascending flat positions
  * (rows = pos / in_features), the derivation HelixLinear does at load
  * (helix_substrate/helix_linear.py:196-203,960-997).  positions, rowptr and
