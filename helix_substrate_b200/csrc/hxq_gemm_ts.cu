@@ -6,35 +6,42 @@
 // not like a GEMM: everything that is not a lookup is kept off the instruction stream of the warps
 // that do the lookups.
 //
-//   * CTA tile: 128 output rows x BN tokens (BN = 16, 32, 64, 128), K walked in stages of one or two
-//     128-column boxes (two up to 64 tokens), one CTA per SM; small row-tile grids split K over
-//     gridDim.z (fp32 partials + a fixed-order sum).
-//   * index bytes: the 512 dequantising threads copy each stage's 128 x 128 box themselves with two
-//     16-byte asynchronous copies per thread (eight lanes per 128-byte line: whole lines per request)
-//     into a ring of up to eight 16 KB boxes laid out in the 128-byte swizzle, up to seven stages
-//     (112 KB per SM) ahead: that much in flight is what this access pattern needs to run near the
-//     DRAM rate.  Each thread's copies report to the box's mbarrier (cp.async.mbarrier.arrive); a
-//     second barrier per box, one arrival per warp, says the codes are in registers and the box may
-//     be refilled.  The warps are not otherwise synchronised: one named barrier per stage over all
-//     512 threads instead was 15 % slower (every stage then takes as long as its slowest warp).
-//   * scale and offset: the 128 rows' values for four stages at a time ride with the index copies
-//     (one 16-byte copy per row and table) into the unused halves of the codebook table's rows.
-//   * warp 0, one lane: TMA producer of the activation tiles (two 64-column boxes of bf16 per stage,
-//     128-byte swizzled, ring of three to six).  No multicast, no cluster.
-//   * warps 2..17: dequantisers, ONE THREAD PER OUTPUT ROW and 32-column quarter of the stage.  A
-//     thread reads its row's 32 codes with two conflict-free 16-byte loads (the swizzle spreads eight
-//     rows over all banks), looks each up in the lane-replicated codebook (one byte-permute + one
-//     load per weight, bank == lane), applies its (row, group) scale and offset in fp32, adds the
-//     row's sidecar deltas that fall into its columns, packs pairs to bf16 and stores its 16
-//     registers straight into the A operand's columns of tensor memory (tcgen05.st 32x32b: TMEM
-//     lane == output row).  The store of a stage is waited for after the lookups of the next one.
-//     The sidecar cursor is thread-local: no cross-lane step anywhere.  (Adding the sidecar term in
-//     the epilogue instead - delta times the activation at its column, per token - was tried: every
-//     such load is a cache-line look-up per lane, 13 us per tile at 32 tokens and 44 us at 128.)
+//   * CTA tile: 128 output rows x BN tokens (BN = 16, 32, 64, 128), K walked in boxes of 128 columns, one
+//     CTA per SM; small row-tile grids split K over gridDim.z (fp32 partials + a fixed-order sum).
+//   * sixteen dequantising warps (2..17): four per TMEM lane quarter, ONE THREAD PER OUTPUT ROW, and each
+//     of the four takes a contiguous quarter of the CTA's K range, a whole box at a time; the MMAs take
+//     the quarters' boxes in turn.  So a thread does what it does once per box - scale and offset (a
+//     16-byte load for four boxes), ring and barrier bookkeeping, the hand-over - once per 128 weights,
+//     and a warp reads only index bytes that it copied itself.  (With the four warps of a quarter on 32
+//     columns each of every box, that was paid once per 32 or 64 weights, and the boxes, copied by
+//     all threads together, needed two more barriers each.)
+//   * index bytes: 16-byte asynchronous copies, four lanes per row's 64 bytes, into the warp's ring of
+//     three or four half boxes (2 KB each), waited for with the warp's own copy groups.
+//   * per weight one byte-permute (code -> shared address) and one load from the lane-replicated codebook
+//     (bank == lane); per pair one packed fp32 FMA (scale, offset) and one pack to bf16; 32 columns go
+//     with one tcgen05.st 32x32b straight into the A operand's columns of tensor memory (TMEM lane ==
+//     output row).  That body is kept in a loop: unrolled four times, with the sidecar's patch in each,
+//     the warps' code did not fit the instruction caches (18 % of the stall cycles).
+//   * sidecar: a thread-local cursor; a box's entries are patched in tensor memory when the box is
+//     complete.  (Adding the sidecar term in the epilogue instead - delta times the activation at its
+//     column, per token - was tried: every such load is a cache-line look-up per lane, 13 us per tile at
+//     32 tokens and 44 us at 128.)
+//   * warp 0, one lane: TMA producer of the activation tiles (two 64-column boxes of bf16 per step,
+//     128-byte swizzled, ring of two to four).  No multicast, no cluster.
 //   * warp 1, one lane: issues tcgen05.mma kind::f16 with A from tensor memory and B (activations,
 //     K-major, 128-byte swizzle) from shared memory into the fp32 accumulator in tensor memory, and
 //     commits the stage, which frees its activation tile and its A columns.
 //   * epilogue (the dequantising warps): accumulator -> registers, + bias, store.
+//
+// Launched dependent (griddepcontrol): the table, the first index boxes and the cursors are set up while
+// the previous kernel drains, where it leaves SMs free.
+//
+// Measured (us, graph replay, this layout / the one of 32-column slices and shared boxes):
+//   tokens                        5           32          64          128
+//   gate [18944 x 3584]           28.9 / 39.5 29.3 / 39.4 30.1 / 39.4 32.0 / 46.9
+//   down [3584 x 18944], K split  40.5 / 47.9 40.3 / 48.0 41.7 / 48.6 44.2 / 58.8
+//   q [3584 x 3584], K split      15.8 / 18.6 16.1 / 19.1 18.0 / 19.7 20.3 / 24.5
+// Bound by the instruction stream of the lookups (about 6 instructions per weight) at 44 % issue.
 //
 // Every mbarrier wait is clock-bounded; a wait that gives up raises a CTA-wide abort flag and the
 // global status word (HXQ_E_TIMEOUT); every other wait of the CTA then returns at its next poll,
@@ -59,10 +66,8 @@ namespace gemmts {
 constexpr int BM = 128;             // output rows per CTA = UMMA M = TMEM lanes
 constexpr int KS = 128;             // K columns per index box (a stage is one or two boxes, see Rings)
 constexpr int DEQ_WARPS = 16;       // four warps per TMEM lane quarter, each takes 32 of a stage's 128 columns
-constexpr int DEQ_THREADS = 32 * DEQ_WARPS;
 constexpr int NUM_THREADS = 32 * (2 + DEQ_WARPS);   // activation producer, MMA issuer, 16 dequantisers
 constexpr int LUT_BYTES = 256 * 256;            // entry c, lane l at c * 256 + l * 4, base on a 64 KB boundary
-constexpr int IDX_BYTES = BM * KS;              // 16 KB per box
 constexpr int SMEM_TOTAL = 232448;
 constexpr int TMEM_COLS = 512;
 constexpr int A_COLS = KS / 2;                  // 64 columns of packed bf16 pairs per box
@@ -120,215 +125,177 @@ __device__ __forceinline__ uint32_t add_to_half(uint32_t pair, int hi, float del
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// Per token tile: H index boxes (128 columns each) per stage, NB activation tiles / A-operand column
-// blocks, NI index boxes-of-a-stage.  Up to 64 tokens a stage is two boxes: what a thread does once
-// per stage (barrier polls, the hand-over to the MMA warp, ring bookkeeping) is then paid once per
-// 64 instead of 32 weights, and the two boxes' lookups overlap each other's tails (at 64 tokens
-// even with rings of two: 76 vs 89 us); at 128 tokens the activation tiles leave no room for that.
-// The table sits on a 64 KB boundary of the shared window, which leaves ~63 KB below and ~100 KB above it.
+// Two neighbouring lookups of one index word as a packed pair (see hxq_gemv.cu).
+__device__ __forceinline__ uint64_t lut_pair(uint32_t word, uint32_t lane_key, int k0) {
+    const uint32_t a0 = __byte_perm(word, lane_key, 0x7604u | (uint32_t)(k0 << 4));
+    const uint32_t a1 = __byte_perm(word, lane_key, 0x7604u | (uint32_t)((k0 + 1) << 4));
+    uint64_t r;
+    asm volatile("{\n\t.reg .f32 lo, hi;\n\tld.shared.f32 lo, [%1];\n\tld.shared.f32 hi, [%2];\n\t"
+                 "mov.b64 %0, {lo, hi};\n\t}" : "=l"(r) : "r"(a0), "r"(a1));
+    return r;
+}
+// bf16x2(c0 * s + t, c1 * s + t): one packed fp32 FMA, each half rounded like fmaf.
+__device__ __forceinline__ uint32_t affine_pack(uint64_t c, uint64_t s2, uint64_t t2) {
+    uint32_t r;
+    asm("{\n\t.reg .b64 v;\n\t.reg .f32 lo, hi;\n\t"
+        "fma.rn.f32x2 v, %1, %2, %3;\n\tmov.b64 {lo, hi}, v;\n\t"
+        "cvt.rn.bf16x2.f32 %0, hi, lo;\n\t}" : "=r"(r) : "l"(c), "l"(s2), "l"(t2));
+    return r;
+}
+__device__ __forceinline__ uint64_t twice(float v) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+
+// Per token tile: NB activation tiles, NA A-operand slots (64 columns each) and R half boxes per
+// dequantising warp.  The table sits on a 64 KB boundary of the shared window, which leaves ~63 KB
+// below and 100 KB above it: the activation tiles go below while they fit, then above, the warps'
+// rings into what is left.
 template <int BN> struct Rings;
-template <> struct Rings<16> { static constexpr int NB = 3, NI = 4, H = 2; };
-template <> struct Rings<32> { static constexpr int NB = 3, NI = 3, H = 2; };
-template <> struct Rings<64> { static constexpr int NB = 2, NI = 2, H = 2; };
-template <> struct Rings<128> { static constexpr int NB = 3, NI = 3, H = 1; };
-static int halves_of(int BN) { return BN <= 64 ? 2 : 1; }
+template <> struct Rings<16> { static constexpr int NB = 4, NA = 7, R = 4; };
+template <> struct Rings<32> { static constexpr int NB = 3, NA = 7, R = 4; };
+template <> struct Rings<64> { static constexpr int NB = 3, NA = 7, R = 3; };
+template <> struct Rings<128> { static constexpr int NB = 2, NA = 6, R = 3; };
+constexpr int HALF_BYTES = 32 * 64;         // a warp's half box: 32 rows x 64 codes
 
 template <int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap map_x, const Args a) {
-    constexpr int H = Rings<BN>::H;                      // index boxes per stage
-    constexpr int KST = KS * H;                          // K columns per stage
-    constexpr int B_BYTES = BN * KST * 2;                // 2 H [BN x 64] bf16 sub-tiles
-    constexpr int IDXB = IDX_BYTES * H;                  // index bytes per stage
-    constexpr int ACOLS = A_COLS * H;                    // A-operand columns per stage
-    constexpr int NB = Rings<BN>::NB;
-    constexpr int NI = Rings<BN>::NI;
-    // stages the index copies run ahead: one box of slack where the ring is deep enough, so that a warp
-    // can start the next stage while the slowest warp is still reading the previous one
-    constexpr int PD = NI >= 5 ? NI - 2 : NI - 1;
-    static_assert((BN < 32 ? 32 : BN) + NB * ACOLS <= TMEM_COLS, "accumulator + A ring must fit tensor memory");
-    static_assert(NI >= 2 && NI <= 8 && NB >= 2 && NB <= 6, "barrier and slot-table layout");
+    constexpr int B_BYTES = BN * KS * 2;                 // two [BN x 64] bf16 sub-tiles
+    constexpr int NB = Rings<BN>::NB, NA = Rings<BN>::NA, R = Rings<BN>::R;
+    constexpr uint32_t RING = R * HALF_BYTES;
+    static_assert((BN < 32 ? 32 : BN) + NA * A_COLS <= TMEM_COLS, "accumulator + A ring must fit tensor memory");
+    static_assert(NB <= 8 && NA <= 8, "barrier layout");
     extern __shared__ __align__(1024) char smem_raw[];
     const uint32_t smem_base = sm100::smem_u32(smem_raw);
     const uint32_t lut_base = (smem_base + 0xFFFFu) & ~0xFFFFu;
     char* lut = smem_raw + (lut_base - smem_base);
-    // Two rings share what is left of shared memory around the table: the larger items first, below
-    // the table while they fit there, then the smaller ones in what is left below, the rest above.
     const uint32_t lo0 = (smem_base + 1023u) & ~1023u;
     const uint32_t hi0 = lut_base + LUT_BYTES;
-    constexpr bool B_FIRST = B_BYTES > IDXB;
-    constexpr uint32_t SZ1 = B_FIRST ? B_BYTES : IDXB, SZ2 = B_FIRST ? IDXB : B_BYTES;
-    constexpr int N1 = B_FIRST ? NB : NI, N2 = B_FIRST ? NI : NB;
-    const int room_lo = (int)(lut_base - lo0);
-    const int n1_lo = room_lo / (int)SZ1 < N1 ? room_lo / (int)SZ1 : N1;
-    const int n2_lo = (room_lo - n1_lo * (int)SZ1) / (int)SZ2 < N2 ? (room_lo - n1_lo * (int)SZ1) / (int)SZ2 : N2;
-    const uint32_t lo2 = lo0 + (uint32_t)n1_lo * SZ1, hi2 = hi0 + (uint32_t)(N1 - n1_lo) * SZ1;
-    const bool layout_ok = hi2 + (uint32_t)(N2 - n2_lo) * SZ2 <= smem_base + SMEM_TOTAL;
-    auto slot1 = [&](int i) -> uint32_t { return i < n1_lo ? lo0 + (uint32_t)i * SZ1 : hi0 + (uint32_t)(i - n1_lo) * SZ1; };
-    auto slot2 = [&](int i) -> uint32_t { return i < n2_lo ? lo2 + (uint32_t)i * SZ2 : hi2 + (uint32_t)(i - n2_lo) * SZ2; };
-    auto b_slot = [&](int i) -> uint32_t { return B_FIRST ? slot1(i) : slot2(i); };       // activation tile i
-    auto idx_slot = [&](int i) -> uint32_t { return B_FIRST ? slot2(i) : slot1(i); };     // index box i
+    const int fit = (int)(lut_base - lo0) / B_BYTES;
+    const int nb_lo = fit < NB ? fit : NB;                                   // activation tiles below the table
+    auto b_slot = [&](int i) -> uint32_t { return i < nb_lo ? lo0 + (uint32_t)(i * B_BYTES) : hi0 + (uint32_t)((i - nb_lo) * B_BYTES); };
+    const uint32_t lo1 = lo0 + (uint32_t)(nb_lo * B_BYTES), hi1 = hi0 + (uint32_t)((NB - nb_lo) * B_BYTES);
+    const int nr_lo = (int)((lut_base - lo1) / RING) < DEQ_WARPS ? (int)((lut_base - lo1) / RING) : DEQ_WARPS;   // warps' rings below it
+    const bool layout_ok = hi1 + (uint32_t)(DEQ_WARPS - nr_lo) * RING <= smem_base + SMEM_TOTAL;
     // barriers live in the unused upper halves of the table's first rows
-    uint64_t* b_full = reinterpret_cast<uint64_t*>(lut + 128);       // [NB] activation tile landed
-    uint64_t* a_full = b_full + 6;                                   // [NB] A columns of the stage written
-    uint64_t* st_free = reinterpret_cast<uint64_t*>(lut + 256 + 128);// [NB] MMAs of the stage retired
-    uint64_t* acc_full = st_free + 6;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(st_free + 7);
+    uint64_t* b_full = reinterpret_cast<uint64_t*>(lut + 128);            // [NB] activation tile landed
+    uint64_t* b_free = b_full + 8;                                        // [NB] MMAs that read it retired
+    uint64_t* a_full = reinterpret_cast<uint64_t*>(lut + 256 + 128);      // [NA] A columns of the box written
+    uint64_t* a_free = a_full + 8;                                        // [NA] MMAs that read them retired
+    uint64_t* acc_full = reinterpret_cast<uint64_t*>(lut + 512 + 128);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    uint64_t* idx_full = reinterpret_cast<uint64_t*>(lut + 512 + 128);   // [NI] index box landed (every copying thread reports)
-    uint64_t* idx_free = idx_full + 8;                                   // [NI] codes read by all dequantising warps
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * BN;
     const int o0 = blockIdx.y * BM;
+    // this CTA's boxes [KS0, KS0 + NK), in four contiguous parts, one per group of four warps; the
+    // MMAs take the parts' boxes in turn: step i is box i / 4 of part i % 4
     const int KS0 = blockIdx.z * a.k_per_split;
     const int NK = (a.k_steps - KS0 < a.k_per_split) ? a.k_steps - KS0 : a.k_per_split;
+    auto part_first = [&](int q) -> int { return KS0 + q * (NK >> 2) + (q < (NK & 3) ? q : (NK & 3)); };
 
-    // ---- the dequantising threads (warps 2..17; the definitions below are only used by them)
+    // ---- the dequantising warps (2..17; the definitions below are only used by them)
     const int dw = warp - 2;
-    const int dt = threadIdx.x - 64;              // 0 .. 511
     const int quarter = warp & 3;                 // TMEM lanes this warp may touch: [32 * quarter, +32)
-    const int kq = dw >> 2;                       // which 32 columns of each stage (warps 2..17: every quarter gets kq = 0..3 once)
-    const int r = 32 * quarter + lane;            // row inside the CTA tile == TMEM lane
-    const int row = o0 + r;
+    const int kq = dw >> 2;                       // its part of the K range (warps 2..17: every quarter gets 0..3 once)
+    const int row = o0 + 32 * quarter + lane;     // this thread's output row
     const bool row_ok = row < a.out_features;
     const bool affine = a.group_size > 0;
+    const int box0 = part_first(kq);
+    const int n_box = (NK >> 2) + (kq < (NK & 3) ? 1 : 0);
+    const int n_half = 2 * n_box;
+    const uint32_t ring = dw < nr_lo ? lo1 + (uint32_t)dw * RING : hi1 + (uint32_t)(dw - nr_lo) * RING;
 
-    // ---- scale / offset of (row, this thread's 32 columns of a box)
-    // Staged case (one group per box, fp32 tables with 16-byte aligned rows - every Qwen2.5 shape):
-    // the 128 rows' values for FOUR boxes at a time ride with the index copies as one 16-byte
-    // asynchronous copy per row and table into the unused halves of the codebook table's rows
-    // (two buffers), and a thread picks its row's four values up with one 16-byte shared load.
-    // A per-thread global load instead costs 32 cache-line look-ups per warp instruction, twice per
-    // stage, on the same load/store pipe as the table lookups: it doubled the stage time.
-    // Other layouts (fp16 tables, odd group sizes, shards starting mid-row-of-four) load per thread.
-    // (a K slice must start on a block of four boxes: with two buffers, the third block's copy would
-    // otherwise be issued in the prologue, before the first block has been read)
-    const bool st_staged = affine && a.group_size == KS && a.col0 % KS == 0 && a.st_dtype == HXQ_F32 &&
-                           a.ld_st % 4 == 0 && ((KS0 * H) & 3) == 0 &&
-                           ((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(a.offsets)) & 15) == 0;
-    const int g_base = affine ? a.col0 / a.group_size : 0;
-    // hole h (16 bytes) of buffer b: entries [b][table][row], eight per table row, from table row 8 on
-    auto st_hole = [&](int b, int which, int rr) -> uint32_t {
-        const int h = b * 256 + which * 128 + rr;
-        return lut_base + (uint32_t)((8 + (h >> 3)) * 256 + 128 + (h & 7) * 16);
-    };
-    const int sf_row = dt & 127, sf_which = (dt >> 7) & 1;       // fetch mapping (threads 0..255)
-    const bool sf_ok = st_staged && dt < 256 && o0 + sf_row < a.out_features;
-    const float* sf_src = reinterpret_cast<const float*>(sf_which ? a.offsets : a.scales) +
-                          (int64_t)(sf_ok ? o0 + sf_row : 0) * a.ld_st;
-    auto fetch_st4 = [&](int kj) {     // groups 4 B .. 4 B + 3 of the block B that stage kj's first box belongs to
-        if (st_staged && dt < 256) {
-            const int blk = ((KS0 + kj) * H) >> 2;
-            int n = a.n_groups - 4 * blk;
-            n = n > 4 ? 4 : (n < 0 ? 0 : n);
-            const uint32_t bytes = sf_ok ? (uint32_t)(4 * n) : 0u;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;"
-                         :: "r"(st_hole(blk & 1, sf_which, sf_row)), "l"(bytes ? sf_src + 4 * blk : reinterpret_cast<const float*>(a.scales)), "r"(bytes) : "memory");
-        }
-    };
-    auto load_st = [&](int bx, float& s, float& t) {     // the per-thread path; bx: box number inside this K slice
-        s = 1.f; t = 0.f;
-        if (affine && row_ok) {
-            int g = (a.col0 + (KS0 * H + bx) * KS + kq * 32) / a.group_size - g_base;
-            g = g < a.n_groups ? g : a.n_groups - 1;      // K tail: those activations are zero
-            const int64_t o = (int64_t)row * a.ld_st + g;
-            if (a.st_dtype == HXQ_F32) {
-                s = reinterpret_cast<const float*>(a.scales)[o];
-                t = reinterpret_cast<const float*>(a.offsets)[o];
-            } else {
-                s = __half2float(reinterpret_cast<const __half*>(a.scales)[o]);
-                t = __half2float(reinterpret_cast<const __half*>(a.offsets)[o]);
-            }
-        }
-    };
-
-    // ---- index copies.  Copy mapping (not the row this thread dequantises), per box: chunk q = dt + 512 c,
-    // c = 0, 1: box row q / 8, 16-byte piece q % 8 -> eight consecutive lanes fetch one 128-byte line.
-    const int c_row = dt >> 3, c_piece = dt & 7;                 // second copy: row + 64, same piece
-    const bool c_ok0 = o0 + c_row < a.out_features, c_ok1 = o0 + c_row + 64 < a.out_features;
-    const uint8_t* c_src0 = a.idx + (int64_t)(c_ok0 ? o0 + c_row : 0) * a.ld_idx + (int64_t)KS0 * KST + c_piece * 16;
-    const uint8_t* c_src1 = a.idx + (int64_t)(c_ok1 ? o0 + c_row + 64 : 0) * a.ld_idx + (int64_t)KS0 * KST + c_piece * 16;
-    const uint32_t c_dst0 = (uint32_t)(c_row * 128) + ((uint32_t)(c_piece ^ (c_row & 7)) << 4);
-    const uint32_t c_dst1 = c_dst0 + 64u * 128u;                 // (row + 64) & 7 == row & 7
-    // stages whose columns all lie inside the matrix; the copies of later ones are cut at the edge
-    const int full_stages = a.in_features / KST - KS0;
-    auto copy_stage = [&](int kj) {     // this thread's 2 H pieces of stage kj into ring slot kj % NI
-        if (kj < NK) {
-            if (kj == 0 || (((KS0 + kj) * H) & 3) == 0) fetch_st4(kj);
-            const uint32_t slot = idx_slot(kj % NI);
+    // ---- index copies: a warp copies the 32 x 64 half boxes that it reads itself, four lanes per
+    // row's 64 bytes, eight rows per instruction; 16-byte piece c of row r at r * 64 + (c ^ (r / 2 & 3)) * 16,
+    // so that eight lanes reading the same piece of their own rows meet no bank twice
+    const int c_row = lane >> 2, c_piece = lane & 3;
+    const uint32_t c_dst = (uint32_t)(c_row * 64 + ((c_piece ^ ((c_row >> 1) & 3)) << 4));   // (row + 8 has the same swizzle)
+    const int c_rows = a.out_features - (o0 + 32 * quarter + c_row);        // rows of this lane's column that exist, by eight
+    const int64_t c_k0 = (int64_t)box0 * KS + c_piece * 16;
+    const uint8_t* c_src = a.idx + (int64_t)(c_rows > 0 ? o0 + 32 * quarter + c_row : 0) * a.ld_idx + c_k0;
+    auto copy_half = [&](int q, uint32_t slot) {      // half box q of this warp; always one group
+        if (q < n_half) {
+            const bool in_k = c_k0 + 64 * q < a.in_features;       // (in_features is a multiple of 16)
 #pragma unroll
-            for (int h = 0; h < H; ++h) {
-                const int64_t off = (int64_t)kj * KST + h * KS;
-                const bool in_k = kj < full_stages || (int64_t)KS0 * KST + off + c_piece * 16 + 16 <= a.in_features;
+            for (int i = 0; i < 4; ++i) {
                 // rows past the matrix and columns past its end are filled with zeros (source size 0)
-                const uint32_t n0 = (c_ok0 && in_k) ? 16u : 0u, n1 = (c_ok1 && in_k) ? 16u : 0u;
-                const uint32_t box = slot + (uint32_t)(h * IDX_BYTES);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(box + c_dst0), "l"(n0 ? c_src0 + off : a.idx), "r"(n0) : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(box + c_dst1), "l"(n1 ? c_src1 + off : a.idx), "r"(n1) : "memory");
+                const uint32_t n = (in_k && 8 * i < c_rows) ? 16u : 0u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                             :: "r"(ring + slot + c_dst + (uint32_t)(i * 512)), "l"(n ? c_src + 64 * q + (int64_t)(8 * i) * a.ld_idx : a.idx), "r"(n) : "memory");
             }
-            // one of the stage barrier's 512 expected arrivals, made when this thread's copies so far have landed
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(sm100::smem_u32(&idx_full[kj % NI])) : "memory");
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NB; ++s) {
             sm100::mbar_init(&b_full[s], 1);
-            sm100::mbar_init(&a_full[s], DEQ_WARPS);
-            sm100::mbar_init(&st_free[s], 1);
+            sm100::mbar_init(&b_free[s], 1);
         }
-        for (int s = 0; s < NI; ++s) {
-            sm100::mbar_init(&idx_full[s], DEQ_THREADS);
-            sm100::mbar_init(&idx_free[s], DEQ_WARPS);
+        for (int s = 0; s < NA; ++s) {
+            sm100::mbar_init(&a_full[s], 4);
+            sm100::mbar_init(&a_free[s], 1);
         }
         sm100::mbar_init(acc_full, 1);
         *abort_flag = 0;
         sm100::fence_barrier_init();
         sm100::prefetch_tensormap(&map_x);
     }
-    // ---- sidecar of this row tile: the CSR entries of rows o0 .. o0 + 127 are one contiguous run of
-    // cols[] / deltas[]; up to SC_MAX of them are copied into the table's unused halves (rows 72 ..),
-    // so that the per-thread cursors below read shared memory.  (Cursors on global memory made every
-    // warp wait, once per stage, for the DRAM miss of the previous stage's cursor refill: that wait,
-    // not the lookups, set the stage time.)  A tile with more entries keeps its cursors on global memory.
-    constexpr int SC_MAX = 2944, SC_ROW_C = 72, SC_ROW_D = SC_ROW_C + SC_MAX / 32;   // (0.1 % of 128 x 18944 weights is 2425)
-    static_assert(SC_ROW_D + SC_MAX / 32 <= 256, "sidecar staging must fit the table's rows");
-    int sc_e0 = 0, sc_n = 0;
-    if (a.rowptr != nullptr) {
-        const int o1 = o0 + BM < a.out_features ? o0 + BM : a.out_features;
-        sc_e0 = a.rowptr[o0];
-        sc_n = a.rowptr[o1] - sc_e0;
-    }
-    const bool sc_staged = sc_n <= SC_MAX;
-    auto sc_addr = [&](int base_row, int e) -> uint32_t {     // entry e (relative to the tile's first)
-        return lut_base + ((uint32_t)(base_row + (e >> 5)) << 8) + 128u + ((uint32_t)(e & 31) << 2);
-    };
-    __syncthreads();          // barriers initialised
-    // The first index boxes are asked for before the rest is set up: the table build and the
-    // tensor-memory allocation below overlap their flight (they touch neither the ring slots nor the
-    // table's holes the scale/offset values go to).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // The first half boxes are asked for before the rest is set up: the table build and the
+    // tensor-memory allocation below overlap their flight.
     if (layout_ok && warp >= 2) {
-        if (sc_staged) {     // (these copies are covered by the first box's barrier arrival below)
-            for (int e = dt; e < sc_n; e += DEQ_THREADS) {
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(sc_addr(SC_ROW_C, e)), "l"(a.cols + sc_e0 + e) : "memory");
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(sc_addr(SC_ROW_D, e)), "l"(a.deltas + sc_e0 + e) : "memory");
-            }
-        }
 #pragma unroll
-        for (int kj = 0; kj < PD; ++kj) copy_stage(kj);
+        for (int q = 0; q < R - 1; ++q) copy_half(q, (uint32_t)(q * HALF_BYTES));
     }
     if (warp == 1) {
         sm100::tmem_alloc(tmem_slot, TMEM_COLS);
         sm100::tmem_relinquish();
     }
-    // lane-replicated codebook (the lower 128 bytes of each 256-byte row)
-    for (int i = threadIdx.x; i < 256 * 32; i += NUM_THREADS)
-        *reinterpret_cast<float*>(lut + (i >> 5) * 256 + (i & 31) * 4) = a.cb[i >> 5];
+    // lane-replicated codebook (the lower 128 bytes of each 256-byte row), a warp's entries all asked for at once
+    {
+        constexpr int PER = (256 + NUM_THREADS / 32 - 1) / (NUM_THREADS / 32);
+        float c[PER];
+#pragma unroll
+        for (int j = 0; j < PER; ++j) c[j] = warp + j * (NUM_THREADS / 32) < 256 ? a.cb[warp + j * (NUM_THREADS / 32)] : 0.f;
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+            if (warp + j * (NUM_THREADS / 32) < 256) *reinterpret_cast<float*>(lut + (warp + j * (NUM_THREADS / 32)) * 256 + lane * 4) = c[j];
+    }
+    // ---- sidecar cursor of this thread's row inside its part of K: entries are sorted by column; the next two are
+    // held, so that the load that refills them is not waited for when one is used.  Started here, in the shadow
+    // of the first boxes' flight, and with the last 16 candidates in one round of loads: a chain of
+    // dependent cache misses down to one entry held every CTA up for 4 us before its first lookup.
+    int e_cur = 0, e_end = 0, nc = 0x7fffffff, nc1 = 0x7fffffff;
+    float nd = 0.f, nd1 = 0.f;
+    if (layout_ok && warp >= 2 && a.rowptr != nullptr && row_ok && n_half > 0) {
+        e_cur = a.rowptr[row];
+        e_end = a.rowptr[row + 1];
+        if (box0 > 0) {
+            const int k0 = box0 * KS;
+            int hi = e_end;
+            while (hi - e_cur > 16) {
+                const int mid = (e_cur + hi) >> 1;
+                if (a.cols[mid] < k0) e_cur = mid + 1; else hi = mid;
+            }
+            int below = 0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) below += (e_cur + j < hi && a.cols[e_cur + j] < k0) ? 1 : 0;
+            e_cur += below;
+        }
+        if (e_cur < e_end) { nc = a.cols[e_cur]; nd = a.deltas[e_cur]; }
+        if (e_cur + 1 < e_end) { nc1 = a.cols[e_cur + 1]; nd1 = a.deltas[e_cur + 1]; }
+    }
     sm100::tc_fence_before_sync();
     __syncthreads();
     sm100::tc_fence_after_sync();
+    // everything above reads weights only; activations, results and partials belong to the stream's earlier kernels until here
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_a0 = tmem_base + (uint32_t)(BN < 32 ? 32 : BN);   // the A ring follows the accumulator's columns
 
@@ -338,20 +305,20 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_x, const Args a) {
         // ------------------------------------------------------------ activation producer (TMA)
         if (lane == 0) {
             int armed = 0;
-            for (int ks = 0; ks < NK; ++ks) {
-                const int s = ks % NB;
-                const uint32_t ph = (uint32_t)(ks / NB) & 1u;
-                if (!sm100::mbar_wait(&st_free[s], ph ^ 1u, abort_flag, 2000000000LL, 200u)) break;
+            for (int i = 0; i < NK; ++i) {
+                const int s = i % NB;
+                if (!sm100::mbar_wait(&b_free[s], ((uint32_t)(i / NB) & 1u) ^ 1u, abort_flag, 2000000000LL, 100u)) break;
                 char* bt = smem_raw + (b_slot(s) - smem_base);
+                const int k = (part_first(i & 3) + (i >> 2)) * KS;
                 sm100::mbar_arrive_expect_tx(&b_full[s], (uint32_t)B_BYTES);
 #pragma unroll
-                for (int j = 0; j < 2 * H; ++j)       // 64-column sub-tiles
-                    sm100::tma_load_2d(bt + j * (BN * 128), &map_x, &b_full[s], (KS0 + ks) * KST + 64 * j, m0);
-                armed = ks + 1;
+                for (int j = 0; j < 2; ++j)           // 64-column sub-tiles
+                    sm100::tma_load_2d(bt + j * (BN * 128), &map_x, &b_full[s], k + 64 * j, m0);
+                armed = i + 1;
             }
             if (*abort_flag != 0) {
-                for (int ks = (armed > NB ? armed - NB : 0); ks < armed; ++ks)
-                    sm100::mbar_wait(&b_full[ks % NB], (uint32_t)(ks / NB) & 1u, abort_flag, 200000000LL);
+                for (int i = (armed > NB ? armed - NB : 0); i < armed; ++i)
+                    sm100::mbar_wait(&b_full[i % NB], (uint32_t)(i / NB) & 1u, abort_flag, 200000000LL);
             }
         }
     } else if (warp == 1) {
@@ -359,179 +326,151 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_x, const Args a) {
         if (lane == 0) {
             constexpr uint32_t idesc = sm100::make_idesc_bf16(BM, BN);
             bool ok = true;
-            for (int ks = 0; ks < NK && ok; ++ks) {
-                const int s = ks % NB;
-                const uint32_t ph = (uint32_t)(ks / NB) & 1u;
-                ok = sm100::mbar_wait(&b_full[s], ph, abort_flag, 2000000000LL, 50u) && sm100::mbar_wait(&a_full[s], ph, abort_flag, 2000000000LL, 50u);
+            for (int i = 0; i < NK && ok; ++i) {
+                const int s = i % NB, sa = i % NA;
+                ok = sm100::mbar_wait(&b_full[s], (uint32_t)(i / NB) & 1u, abort_flag, 2000000000LL, 50u) &&
+                     sm100::mbar_wait(&a_full[sa], (uint32_t)(i / NA) & 1u, abort_flag, 2000000000LL, 50u);
                 if (!ok) break;
                 sm100::tc_fence_after_sync();
                 // B: sub-tile kk / 4 (64 K columns each), + 32 bytes (2 in descriptor units) per 16-column slice
                 const uint64_t db0 = sm100::make_desc_k_sw128(b_slot(s));
-                const uint32_t ta = tmem_a0 + (uint32_t)(s * ACOLS);
+                const uint32_t ta = tmem_a0 + (uint32_t)(sa * A_COLS);
 #pragma unroll
-                for (int kk = 0; kk < KST / 16; ++kk) {
+                for (int kk = 0; kk < KS / 16; ++kk) {
                     const uint64_t db = db0 + (uint64_t)((kk >> 2) * (BN * 128 / 16) + 2 * (kk & 3));
-                    umma_bf16_ts(tmem_base, ta + (uint32_t)(kk * 8), db, idesc, (ks > 0 || kk > 0) ? 1u : 0u);
+                    umma_bf16_ts(tmem_base, ta + (uint32_t)(kk * 8), db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
                 }
-                sm100::umma_commit(&st_free[s]);
+                sm100::umma_commit(&b_free[s]);
+                sm100::umma_commit(&a_free[sa]);
             }
             if (ok) sm100::umma_commit(acc_full);
         }
     } else {
         // ------------------------------------------------------------ dequantising warps
         const uint32_t lane_key = lut_base | ((uint32_t)lane << 2);
-        const uint32_t t_row = tmem_a0 + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(kq * 16);
+        const uint32_t t_row = tmem_a0 + ((uint32_t)(32 * quarter) << 16);
+        const uint32_t r_src = ring + (uint32_t)(lane * 64);
+        const uint32_t r_swz = (uint32_t)((lane >> 1) & 3);
 
-        // sidecar cursor of this row: entries are sorted by column; this thread takes those inside its
-        // 32 columns of every stage and steps over the others.  e_cur / e_end count from the tile's first
-        // entry; nc is the column of entry e_cur (read when the cursor moves).
-        int e_cur = 0, e_end = 0, nc = 0x7fffffff;
-        if (a.rowptr != nullptr && row_ok) {
-            e_cur = a.rowptr[row] - sc_e0;
-            e_end = a.rowptr[row + 1] - sc_e0;
-        }
-        auto sc_col = [&](int e) -> int {
-            if (sc_staged) {
-                int v;
-                asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(sc_addr(SC_ROW_C, e)));
-                return v;
+        // ---- scale / offset of this thread's row, one pair per half box (group_size and col0 are multiples of 64).
+        // Block case (128-column groups, fp32 tables with 16-byte aligned rows, shard starting on a group - every
+        // Qwen2.5 shape): one 16-byte load each for four boxes, a block ahead; else one pair, a half box ahead.
+        const int g_base = affine ? a.col0 / a.group_size : 0;
+        const bool st_block = affine && a.group_size == KS && a.col0 % KS == 0 && a.st_dtype == HXQ_F32 && a.ld_st % 4 == 0 &&
+                              ((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(a.offsets)) & 15) == 0;
+        const int64_t st_row = (int64_t)(row_ok ? row : 0) * a.ld_st;
+        auto load_block = [&](int blk, float4& s4, float4& t4) {      // groups 4 blk .. 4 blk + 3
+            s4 = make_float4(1.f, 1.f, 1.f, 1.f); t4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int n = a.n_groups - 4 * blk;
+            const float* ps = reinterpret_cast<const float*>(a.scales) + st_row + 4 * blk;
+            const float* pt = reinterpret_cast<const float*>(a.offsets) + st_row + 4 * blk;
+            if (n >= 4) {
+                s4 = *reinterpret_cast<const float4*>(ps);
+                t4 = *reinterpret_cast<const float4*>(pt);
+            } else if (n > 0) {     // last, short block of the row: never past the row's groups
+                s4.x = ps[0]; t4.x = pt[0];
+                if (n > 1) { s4.y = ps[1]; t4.y = pt[1]; }
+                if (n > 2) { s4.z = ps[2]; t4.z = pt[2]; }
             }
-            return a.cols[sc_e0 + e];
         };
-        auto sc_delta = [&](int e) -> float {
-            if (sc_staged) {
-                float v;
-                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(sc_addr(SC_ROW_D, e)));
-                return v;
-            }
-            return a.deltas[sc_e0 + e];
-        };
-        float st_s_n = 1.f, st_t_n = 0.f;
-        if (!st_staged) load_st(0, st_s_n, st_t_n);      // box 0
-        float4 s4 = make_float4(1.f, 1.f, 1.f, 1.f), t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        bool failed = false;          // one of this thread's bounded waits gave up (or saw the abort flag)
-        int stored = -1;              // last stage whose tcgen05.st was issued and not yet handed over
-        auto hand_over = [&]() {      // the pending store has completed: let the MMA warp have the stage
-            tmem_st_wait();
-            sm100::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) sm100::mbar_arrive(&a_full[stored % NB]);
-            stored = -1;
-        };
-        for (int ks = 0; ks < NK; ++ks) {
-            if (ks + PD < NK) {
-                // the box of stage ks + PD held stage ks + PD - NI: wait until every warp has those codes in registers
-                if (ks + PD >= NI && !__all_sync(0xffffffffu, sm100::mbar_wait(&idx_free[(ks + PD) % NI], (uint32_t)((ks + PD) / NI - 1) & 1u, abort_flag))) {
-                    failed = true;
-                    break;
-                }
-                copy_stage(ks + PD);
-            }
-            if (!__all_sync(0xffffffffu, sm100::mbar_wait(&idx_full[ks % NI], (uint32_t)(ks / NI) & 1u, abort_flag))) {
-                failed = true;
-                break;
-            }
-            if (ks == 0) {     // the staged sidecar has landed with the first box: position the cursor
-                const int k_first = KS0 * KST;
-                while (e_cur < e_end && sc_col(e_cur) < k_first) ++e_cur;
-                nc = e_cur < e_end ? sc_col(e_cur) : 0x7fffffff;
-            }
-            const uint32_t slot = idx_slot(ks % NI);
-            const int sb = ks % NB;
-#pragma unroll
-            for (int h = 0; h < H; ++h) {     // the stage's boxes; unrolled, so that the second box's code loads and lookups
-                                              // are scheduled into the first one's patching and store (7 % at 32 tokens)
-                const int bx = ks * H + h;            // box number inside this K slice
-                float sc, of;
-                if (st_staged) {
-                    const int ag = KS0 * H + bx;      // == the box's group number
-                    if (bx == 0 || (ag & 3) == 0) {
-                        const uint32_t hs = st_hole((ag >> 2) & 1, 0, r), ht = st_hole((ag >> 2) & 1, 1, r);
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s4.x), "=f"(s4.y), "=f"(s4.z), "=f"(s4.w) : "r"(hs));
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t4.x), "=f"(t4.y), "=f"(t4.z), "=f"(t4.w) : "r"(ht));
-                    }
-                    const int q = ag & 3;
-                    sc = q == 0 ? s4.x : (q == 1 ? s4.y : (q == 2 ? s4.z : s4.w));
-                    of = q == 0 ? t4.x : (q == 1 ? t4.y : (q == 2 ? t4.z : t4.w));
+        auto load_st = [&](int q, float& s, float& t) {               // half box q of this warp
+            s = 1.f; t = 0.f;
+            if (affine) {
+                int g = (a.col0 + box0 * KS + 64 * q) / a.group_size - g_base;
+                g = g < a.n_groups ? g : a.n_groups - 1;      // K tail: those activations are zero
+                const int64_t o = st_row + g;
+                if (a.st_dtype == HXQ_F32) {
+                    s = reinterpret_cast<const float*>(a.scales)[o];
+                    t = reinterpret_cast<const float*>(a.offsets)[o];
                 } else {
-                    sc = st_s_n; of = st_t_n;
-                    if (bx + 1 < NK * H) load_st(bx + 1, st_s_n, st_t_n);
+                    s = __half2float(reinterpret_cast<const __half*>(a.scales)[o]);
+                    t = __half2float(reinterpret_cast<const __half*>(a.offsets)[o]);
+                }
+            }
+        };
+        float4 s4 = make_float4(1.f, 1.f, 1.f, 1.f), t4 = make_float4(0.f, 0.f, 0.f, 0.f), s4n = s4, t4n = t4;
+        float sc_n = 1.f, of_n = 0.f;
+        if (n_half > 0) {
+            if (st_block) load_block(box0 >> 2, s4n, t4n);
+            else load_st(0, sc_n, of_n);
+        }
+
+        bool failed = false;          // one of this thread's bounded waits gave up (or saw the abort flag)
+        uint32_t slot = 0;
+        for (int j = 0; j < n_box; ++j) {
+            const int i = 4 * j + kq;             // the step this box is
+            const int sa = i % NA;
+            const uint32_t t_dst = t_row + (uint32_t)(sa * A_COLS);
+            if (st_block) {
+                const int g = box0 + j;
+                if (j == 0 || (g & 3) == 0) {
+                    s4 = s4n; t4 = t4n;
+                    if (((g >> 2) + 1) * 4 < box0 + n_box) load_block((g >> 2) + 1, s4n, t4n);
+                }
+                sc_n = (g & 3) == 0 ? s4.x : ((g & 3) == 1 ? s4.y : ((g & 3) == 2 ? s4.z : s4.w));
+                of_n = (g & 3) == 0 ? t4.x : ((g & 3) == 1 ? t4.y : ((g & 3) == 2 ? t4.z : t4.w));
+            }
+            float sc = 1.f, of = 0.f;
+            // 32 columns at a time, NOT unrolled: with the four bodies side by side the eighteen warps' code did not fit
+            // the instruction caches, a fifth of all stall cycles
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                if ((c & 1) == 0) {
+                    const int q = 2 * j + (c >> 1);
+                    asm volatile("cp.async.wait_group %0;" :: "n"(R - 2) : "memory");
+                    __syncwarp();     // half box q has landed for every lane, and every lane has half box q - 1 in registers
+                    copy_half(q + R - 1, slot == 0 ? RING - HALF_BYTES : slot - HALF_BYTES);     // into the slot half box q - 1 had
+                    sc = sc_n; of = of_n;
+                    if (!st_block && q + 1 < n_half) load_st(q + 1, sc_n, of_n);
                 }
                 uint32_t w[8];
-                {
-                    const uint32_t idx_row = slot + (uint32_t)(h * IDX_BYTES + r * 128);
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {     // 16 codes per load: chunk 2 * kq + c of the row, swizzled by the row
-                        const uint32_t addr = idx_row + ((uint32_t)((2 * kq + c) ^ (r & 7)) << 4);
-                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                     : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3]) : "r"(addr));
-                    }
-                }
-                if (h == H - 1) {     // the stage's codes are (on their way) in registers: its boxes can be refilled
-                    __syncwarp();
-                    if (lane == 0) sm100::mbar_arrive(&idx_free[ks % NI]);
-                }
+                for (int k = 0; k < 2; ++k)
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(w[4 * k]), "=r"(w[4 * k + 1]), "=r"(w[4 * k + 2]), "=r"(w[4 * k + 3])
+                                 : "r"(r_src + slot + (((2 * (c & 1) + k) ^ r_swz) << 4)) : "memory");
+                if (c & 1) slot = slot + HALF_BYTES == RING ? 0 : slot + HALF_BYTES;
+                const uint64_t s2 = twice(sc), t2 = twice(of);
                 uint32_t out[16];
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const uint32_t a0 = __byte_perm(w[j >> 2], lane_key, 0x7604u | (uint32_t)((j & 3) << 4));
-                    const uint32_t a1 = __byte_perm(w[j >> 2], lane_key, 0x7604u | (uint32_t)(((j + 1) & 3) << 4));
-                    float v0, v1;
-                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v0) : "r"(a0));
-                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v1) : "r"(a1));
-                    out[j >> 1] = pack_bf16x2(fmaf(v0, sc, of), fmaf(v1, sc, of));
-                }
-                // sidecar entries of this row inside this box: mine are patched into the packed registers
-                // (a jump per entry instead of a dynamically indexed register array), the others skipped
-                {
-                    const int k_lo = (KS0 * H + bx) * KS + kq * 32;
-                    const int k_st = (KS0 * H + bx + 1) * KS;
-                    while (nc < k_st) {
-                        const int j = nc - k_lo;
-                        if (j >= 0 && j < 32) {
-                            const int hi = j & 1;
-                            const float nd = sc_delta(e_cur);
-                            switch (j >> 1) {
-                                case 0: out[0] = add_to_half(out[0], hi, nd); break;
-                                case 1: out[1] = add_to_half(out[1], hi, nd); break;
-                                case 2: out[2] = add_to_half(out[2], hi, nd); break;
-                                case 3: out[3] = add_to_half(out[3], hi, nd); break;
-                                case 4: out[4] = add_to_half(out[4], hi, nd); break;
-                                case 5: out[5] = add_to_half(out[5], hi, nd); break;
-                                case 6: out[6] = add_to_half(out[6], hi, nd); break;
-                                case 7: out[7] = add_to_half(out[7], hi, nd); break;
-                                case 8: out[8] = add_to_half(out[8], hi, nd); break;
-                                case 9: out[9] = add_to_half(out[9], hi, nd); break;
-                                case 10: out[10] = add_to_half(out[10], hi, nd); break;
-                                case 11: out[11] = add_to_half(out[11], hi, nd); break;
-                                case 12: out[12] = add_to_half(out[12], hi, nd); break;
-                                case 13: out[13] = add_to_half(out[13], hi, nd); break;
-                                case 14: out[14] = add_to_half(out[14], hi, nd); break;
-                                default: out[15] = add_to_half(out[15], hi, nd); break;
-                            }
-                        }
-                        ++e_cur;
-                        nc = e_cur < e_end ? sc_col(e_cur) : 0x7fffffff;
-                    }
-                }
-                __syncwarp();
-                if (h == 0) {
-                    // the previous stage's stores have had these lookups to complete
-                    if (stored >= 0) hand_over();
-                    // the A columns of this ring slot are free once the MMAs that read them NB stages ago have retired
+                for (int p = 0; p < 16; ++p)
+                    out[p] = affine_pack(lut_pair(w[p >> 1], lane_key, 2 * (p & 1)), s2, t2);
+                if (c == 0) {
+                    // the slot's columns are free once the MMAs that read them NA steps ago have retired
                     // (warp-uniform outcome: the store below is a whole-warp instruction)
-                    if (ks >= NB && !__all_sync(0xffffffffu, sm100::mbar_wait(&st_free[sb], (uint32_t)(ks / NB - 1) & 1u, abort_flag))) {
+                    if (i >= NA && !__all_sync(0xffffffffu, sm100::mbar_wait(&a_free[sa], (uint32_t)(i / NA - 1) & 1u, abort_flag))) {
                         failed = true;
                         break;
                     }
                     sm100::tc_fence_after_sync();
                 }
-                tmem_st_32x16(t_row + (uint32_t)(sb * ACOLS + h * A_COLS), out);
+                tmem_st_32x16(t_dst + (uint32_t)(16 * c), out);
             }
             if (failed) break;
-            stored = ks;
+            tmem_st_wait();
+            // sidecar entries of these 32 rows inside the box: column by column, read back, patched in the lanes that
+            // have an entry there, and stored again (about four rounds per box at 0.1 %).  A jump into the packed
+            // registers per entry diverged once per entry and chunk and carried sixteen bodies per chunk.
+            const int k_lo = (box0 + j) * KS;
+            for (uint32_t m; (m = __ballot_sync(0xffffffffu, nc < k_lo + KS)) != 0u; ) {
+                const int col = __shfl_sync(0xffffffffu, (nc - k_lo) >> 1, __ffs(m) - 1);
+                uint32_t v;
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(t_dst + (uint32_t)col) : "memory");
+                sm100::tmem_ld_wait();
+                if (nc < k_lo + KS && ((nc - k_lo) >> 1) == col) {
+                    v = add_to_half(v, nc & 1, nd);
+                    ++e_cur;
+                    nc = nc1; nd = nd1;
+                    if (e_cur + 1 < e_end) { nc1 = a.cols[e_cur + 1]; nd1 = a.deltas[e_cur + 1]; } else { nc1 = 0x7fffffff; }
+                }
+                __syncwarp();
+                asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t_dst + (uint32_t)col), "r"(v) : "memory");
+                tmem_st_wait();
+            }
+            sm100::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) sm100::mbar_arrive(&a_full[sa]);
         }
-        if (stored >= 0) hand_over();
         asm volatile("cp.async.wait_all;" ::: "memory");   // (a loop left early must not retire with copies in flight)
 
         // ------------------------------------------------------------ epilogue
@@ -547,6 +486,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_x, const Args a) {
                 for (int c0 = c_lo; c0 < c_lo + COLS_PER_WARP; c0 += 8) {
                     if (m0 + c0 >= a.M) break;           // warp-uniform
                     uint32_t v[8];
+                    __syncwarp();
                     asm volatile(
                         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -637,8 +577,17 @@ static int launch(const CUtensorMap& mx, const Args& a, int grid_m, int grid_o, 
             return HXQ_E_DEVICE;
         attr_set[dev] = true;
     }
-    gemm_ts_kernel<BN><<<dim3(grid_m, grid_o, splits), NUM_THREADS, SMEM_TOTAL, stream>>>(mx, a);
-    return cudaGetLastError() == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_m, grid_o, splits);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = SMEM_TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set-up on SMs that the previous kernel has left
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_weights_on_stream ? 0 : 1;   // weights still being written on this stream: no early start
+    return cudaLaunchKernelEx(&cfg, gemm_ts_kernel<BN>, mx, a) == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
 
 // xb: the activations as bf16 with a 16-byte aligned row stride (the caller converted them if needed);
@@ -659,17 +608,15 @@ int run(const hxq_desc* d, const __nv_bfloat16* xb, int64_t ldxb, int32_t M, voi
     a.group_size = d->group_size; a.ld_st = d->ld_st; a.st_dtype = d->st_dtype;
     a.n_groups = d->group_size > 0 ? (d->col0 + d->in_features - 1) / d->group_size - d->col0 / d->group_size + 1 : 0;
     a.M = M; a.y_dtype = y_dtype;
-    const int H = halves_of(BN), k_boxes = (d->in_features + KS - 1) / KS;
-    a.k_steps = (k_boxes + H - 1) / H;
+    a.k_steps = (d->in_features + KS - 1) / KS;
     const int grid_o = (d->out_features + BM - 1) / BM;
     const int grid_m = (M + BN - 1) / BN;
-    int splits = pick_splits(grid_m, grid_o, k_boxes, sm_count());
+    int splits = pick_splits(grid_m, grid_o, a.k_steps, sm_count());
     a.k_per_split = a.k_steps;
     a.partial = nullptr;
     if (splits > 1 && split_ws && aligned_to(split_ws, 16) &&
         split_ws_bytes >= (size_t)splits * M * d->out_features * sizeof(float)) {
-        const int per_block = 4 / H;      // stages per block of four boxes (scale/offset staging works in such blocks)
-        a.k_per_split = ((a.k_steps + splits - 1) / splits + per_block - 1) / per_block * per_block;
+        a.k_per_split = (a.k_steps + splits - 1) / splits;
         splits = (a.k_steps + a.k_per_split - 1) / a.k_per_split;   // no empty slice
         if (splits > 1) a.partial = reinterpret_cast<float*>(split_ws);
         else a.k_per_split = a.k_steps;                             // one slice after rounding: nothing to split
