@@ -188,132 +188,204 @@ __global__ void rope_append_kernel(const __nv_bfloat16* __restrict__ qkv, int64_
     dst[i + half] = o1;
 }
 
-constexpr int kAttnChunk = 64;     // cache positions per CTA
+constexpr int kAttnChunk = 64;     // unit of the split: a CTA takes span = R * 64 cache positions
 constexpr int kAttnThreads = 128;
 constexpr int kAttnMaxGroup = 8;   // query heads per KV head
 constexpr int kAttnMaxD = 128;
+constexpr int kAttnUnroll = 4;     // positions of a half-warp's step
+constexpr int kAttnStages = 4;     // steps in a warp's ring: three are in flight while one is used
+constexpr int kAttnStageBytes = 2 * kAttnUnroll * 512;      // a warp's step: K and V of 2 * kAttnUnroll positions
+constexpr int kAttnSmemBytes = (kAttnThreads / 32) * kAttnStages * kAttnStageBytes;
 
-// One CTA: positions [c*64, c*64+64) of one (sequence, KV head), all query heads of the group.
-// Writes per (b, query head, chunk): running max m, sum l and the un-normalised output o[D] (fp32).
-__global__ void __launch_bounds__(kAttnThreads) attn_partial_kernel(const __nv_bfloat16* __restrict__ q, int64_t ld_q,
-                                                                    const __nv_bfloat16* __restrict__ k_cache,
-                                                                    const __nv_bfloat16* __restrict__ v_cache,
-                                                                    const int64_t* __restrict__ pos_p, float* __restrict__ part,
-                                                                    int nq, int nkv, int D, int max_len, int n_chunks, float scale) {
-    const int c = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z, t = threadIdx.x;
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t widen2(uint32_t w) { return f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+
+// One CTA: positions [c * span, (c + 1) * span) of one (sequence, KV head), all G query heads of the group.
+// Writes per (b, query head, c): running max m, sum l and the un-normalised output o[D] (fp32).
+//
+// Bound by HBM at large batches (K and V once) and by latency at batch 1.  A half-warp takes one position, a
+// lane 8 of its 128 dimensions, with the G queries' and the G outputs' share of them in registers; K
+// and V rows pass through a ring in shared memory that each lane fills (16-byte asynchronous copies, 256
+// coalesced bytes a row) and reads back for itself, so nothing but its own copies is ever waited for
+// and 12 KB per warp are in flight (loads into registers, four positions at a time, left the memory idle
+// while a step was computed: 58 us at batch 32).  Scores meet over the 16 lanes in a halving butterfly that leaves lane 2 g with head g;
+// the softmax is a running one per half-warp; probabilities return by shuffles.  fp32 throughout.
+// The eight half-warps' sums meet in shared memory at the end.
+// Measured, 28 query and 4 KV heads of 128 behind 2048 positions: 45 us at batch 32 (134 MB of K and V: 3 TB/s; the
+// sixty-odd shuffles and 230 packed FMAs of a step bound it), about 7 us at batch 1.
+// (K and V tiles in shared memory, a score per thread and an output dimension per thread cost nine
+// shared loads per 32 FMAs and eight per seven: 82 us at batch 32 behind 2048 positions, 12 us at
+// batch 1, most of it one tile's copy, scores, softmax and output in series.)
+template <int G>
+__global__ void __launch_bounds__(kAttnThreads, G == 8 ? 2 : 3)
+attn_partial_kernel(const __nv_bfloat16* __restrict__ q, int64_t ld_q, const __nv_bfloat16* __restrict__ k_cache,
+                    const __nv_bfloat16* __restrict__ v_cache, const int64_t* __restrict__ pos_p, float* __restrict__ part,
+                    int nq, int nkv, int D, int max_len, int n_chunks, int span, float scale) {
+    const int c = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sl = lane & 15, half = lane >> 4;
     pdl_enter();
     const int64_t pos = *pos_p;
-    const int p0 = c * kAttnChunk;
+    const int64_t p0 = (int64_t)c * span;
     if (p0 > pos || pos >= max_len) return;
-    const int G = nq / nkv;
-    const int n_valid = (int)((pos - p0 + 1 < kAttnChunk) ? pos - p0 + 1 : kAttnChunk);
+    const int n = (int)(pos - p0 + 1 < span ? pos - p0 + 1 : span);      // positions of this CTA
+    const bool d_ok = 8 * sl < D;
 
-    __shared__ __align__(16) float q_s[kAttnMaxGroup][kAttnMaxD];
-    __shared__ __align__(16) __nv_bfloat16 k_s[kAttnChunk][kAttnMaxD + 8];   // +16 B per row: rows start in different banks
-    __shared__ __align__(16) __nv_bfloat16 v_s[kAttnChunk][kAttnMaxD + 8];
-    __shared__ float s_s[kAttnMaxGroup][kAttnChunk];
-    __shared__ float m_s[kAttnMaxGroup], l_s[kAttnMaxGroup];
-
-    // K tile, then V tile, as two asynchronous copy groups: V lands while the scores are computed
-    const int64_t base = (((int64_t)b * nkv + kvh) * max_len + p0) * D;
-    const int vec_per_row = D / 8;    // 16-byte pieces per row
-    for (int i = t; i < n_valid * vec_per_row; i += kAttnThreads) {
-        const int r = i / vec_per_row, v = i - r * vec_per_row;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(&k_s[r][v * 8])),
-                     "l"(k_cache + base + (int64_t)r * D + v * 8) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int i = t; i < n_valid * vec_per_row; i += kAttnThreads) {
-        const int r = i / vec_per_row, v = i - r * vec_per_row;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(&v_s[r][v * 8])),
-                     "l"(v_cache + base + (int64_t)r * D + v * 8) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    if (t < G * vec_per_row) {   // G * D / 8 <= 128 vectors of q
-        const int g = t / vec_per_row, d = (t - g * vec_per_row) * 8;
-        const uint4 qv = *reinterpret_cast<const uint4*>(q + (int64_t)b * ld_q + (int64_t)(kvh * G + g) * D + d);
+    uint64_t q2[G][4], o2[G][4];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        uint4 qv = make_uint4(0u, 0u, 0u, 0u);
+        if (d_ok) qv = *reinterpret_cast<const uint4*>(q + (int64_t)b * ld_q + (int64_t)(kvh * G + g) * D + 8 * sl);
         float f[8];
         unpack8(qv, f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) q_s[g][d + e] = f[e] * scale;
+        for (int e = 0; e < 4; ++e) {
+            q2[g][e] = f32x2(f[2 * e] * scale, f[2 * e + 1] * scale);
+            o2[g][e] = 0ull;
+        }
     }
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
-
-    // scores: thread (p = t % 64, hg = t / 64) takes query heads hg, hg + 2, ... of position p
-    {
-        const int p = t & (kAttnChunk - 1), hg = t / kAttnChunk;
-        float acc[kAttnMaxGroup / 2];
+    float m = -INFINITY, l = 0.f;          // of head sl / 2 (lanes 2 g and 2 g + 1 agree)
+    const int64_t base = (((int64_t)b * nkv + kvh) * max_len + p0) * D + (d_ok ? 8 * sl : 0);
+    constexpr int U = kAttnUnroll, NS = kAttnStages, STEP = (kAttnThreads / 32) * 2 * U;
+    extern __shared__ __align__(16) char attn_smem[];
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(attn_smem) + (uint32_t)(warp * NS * kAttnStageBytes + lane * 16);
+    auto fetch = [&](int i0, uint32_t slot) {       // always one group
+        if (i0 < n) {
 #pragma unroll
-        for (int j = 0; j < kAttnMaxGroup / 2; ++j) acc[j] = 0.f;
-        if (p < n_valid) {
-            for (int d = 0; d < D; d += 8) {
-                const uint4 kk = *reinterpret_cast<const uint4*>(&k_s[p][d]);
-                const uint32_t w[4] = {kk.x, kk.y, kk.z, kk.w};
-                float kf[8];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    kf[2 * e] = __uint_as_float(w[e] << 16);
-                    kf[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
-                }
-#pragma unroll
-                for (int j = 0; j < kAttnMaxGroup / 2; ++j) {
-                    const int g = hg + 2 * j;
-                    if (g < G) {
-                        const float4 qa = *reinterpret_cast<const float4*>(&q_s[g][d]);
-                        const float4 qb = *reinterpret_cast<const float4*>(&q_s[g][d + 4]);
-                        acc[j] += kf[0] * qa.x + kf[1] * qa.y + kf[2] * qa.z + kf[3] * qa.w
-                                + kf[4] * qb.x + kf[5] * qb.y + kf[6] * qb.z + kf[7] * qb.w;
-                    }
-                }
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + 2 * u + half;
+                const bool ok = d_ok && i < n;      // the rest is filled with zeros (source size 0)
+                const int64_t off = base + (int64_t)(i < n ? i : 0) * D;
+                const uint32_t bytes = ok ? 16u : 0u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(ring + slot + u * 1024), "l"(k_cache + off), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(ring + slot + u * 1024 + 512), "l"(v_cache + off), "r"(bytes) : "memory");
             }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto take = [&](uint32_t addr) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+        return v;
+    };
+    const int first = warp * 2 * U;
 #pragma unroll
-        for (int j = 0; j < kAttnMaxGroup / 2; ++j) {
-            const int g = hg + 2 * j;
-            if (g < G) s_s[g][p] = (p < n_valid) ? acc[j] : -INFINITY;
-        }
-    }
-    __syncthreads();
+    for (int k = 0; k < NS - 1; ++k) fetch(first + k * STEP, (uint32_t)(k * kAttnStageBytes));
 
-    // softmax pieces per head
-    {
-        const int warp = t >> 5, lane = t & 31;
-        for (int g = warp; g < G; g += kAttnThreads / 32) {
-            const float a0 = s_s[g][lane], a1 = s_s[g][lane + 32];
-            float m = fmaxf(a0, a1);
+    uint32_t slot = 0;
+    for (int i0 = first; i0 < n; i0 += STEP) {
+        asm volatile("cp.async.wait_group %0;" :: "n"(NS - 2) : "memory");       // this step has landed (each lane reads only what it copied)
+        fetch(i0 + (NS - 1) * STEP, slot == 0 ? (NS - 1) * kAttnStageBytes : slot - kAttnStageBytes);   // into the slot of the step before
+        const uint32_t at = ring + slot;
+        slot = slot + kAttnStageBytes == NS * kAttnStageBytes ? 0 : slot + kAttnStageBytes;
+        float s[U];
+        float mx = m;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            const float e0 = __expf(a0 - m), e1 = __expf(a1 - m);   // exp(-inf) = 0 for the masked tail
-            float l = e0 + e1;
+        for (int u = 0; u < U; ++u) {
+            const uint4 kr = take(at + u * 1024);
+            const uint64_t k0 = widen2(kr.x), k1 = widen2(kr.y), k2 = widen2(kr.z), k3 = widen2(kr.w);
+            float v8[8];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-            s_s[g][lane] = e0;
-            s_s[g][lane + 32] = e1;
-            if (lane == 0) { m_s[g] = m; l_s[g] = l; }
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-
-    // o[g][d] = sum_p prob[g][p] * V[p][d]; thread t owns dimension d = t (and d + 128 ... if D > 128: not supported)
-    if (t < D) {
-        float o[kAttnMaxGroup];
-#pragma unroll
-        for (int g = 0; g < kAttnMaxGroup; ++g) o[g] = 0.f;
-        for (int p = 0; p < n_valid; ++p) {
-            const float v = bf(v_s[p][t]);
-#pragma unroll
-            for (int g = 0; g < kAttnMaxGroup; ++g)
-                if (g < G) o[g] += s_s[g][p] * v;
-        }
-#pragma unroll
-        for (int g = 0; g < kAttnMaxGroup; ++g)
-            if (g < G) {
-                float* dst = part + (((int64_t)b * nq + kvh * G + g) * n_chunks + c) * (D + 2);
-                dst[2 + t] = o[g];
-                if (t == 0) { dst[0] = m_s[g]; dst[1] = l_s[g]; }
+            for (int g = 0; g < 8; ++g) {
+                v8[g] = 0.f;
+                if (g < G) {
+                    const uint64_t a = fma2(q2[g < G ? g : 0][3], k3, fma2(q2[g < G ? g : 0][2], k2, fma2(q2[g < G ? g : 0][1], k1, mul2(q2[g < G ? g : 0][0], k0))));
+                    float lo, hi;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+                    v8[g] = lo + hi;
+                }
             }
+            // 16 lanes x 8 heads -> lane's head sl / 2
+            const bool b3 = sl & 8, b2 = sl & 4, b1 = sl & 2;
+            float v4[4], v2[2];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v4[e] = (b3 ? v8[4 + e] : v8[e]) + __shfl_xor_sync(0xffffffffu, b3 ? v8[e] : v8[4 + e], 8);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) v2[e] = (b2 ? v4[2 + e] : v4[e]) + __shfl_xor_sync(0xffffffffu, b2 ? v4[e] : v4[2 + e], 4);
+            float v1 = (b1 ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, b1 ? v2[0] : v2[1], 2);
+            v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
+            s[u] = i0 + 2 * u + half < n ? v1 : -INFINITY;
+            mx = fmaxf(mx, s[u]);
+        }
+        const float ref = mx == -INFINITY ? 0.f : mx;      // (nothing seen yet: every exponential below is of -inf)
+        const float corr = __expf(m - ref);
+        l *= corr;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            s[u] = __expf(s[u] - ref);
+            l += s[u];
+        }
+        if (__any_sync(0xffffffffu, mx != m)) {            // a new maximum somewhere: rescale
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const float cg = __shfl_sync(0xffffffffu, corr, (lane & 16) + 2 * g);
+                const uint64_t c2 = f32x2(cg, cg);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o2[g][e] = mul2(o2[g][e], c2);
+            }
+        }
+        m = mx;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint4 vr = take(at + u * 1024 + 512);
+            const uint64_t v0 = widen2(vr.x), v1 = widen2(vr.y), v2 = widen2(vr.z), v3 = widen2(vr.w);
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const float pg = __shfl_sync(0xffffffffu, s[u], (lane & 16) + 2 * g);
+                const uint64_t p2 = f32x2(pg, pg);
+                o2[g][0] = fma2(p2, v0, o2[g][0]);
+                o2[g][1] = fma2(p2, v1, o2[g][1]);
+                o2[g][2] = fma2(p2, v2, o2[g][2]);
+                o2[g][3] = fma2(p2, v3, o2[g][3]);
+            }
+        }
+    }
+
+    // ---- the eight half-warps' (m, l, o) meet
+    constexpr int S = kAttnThreads / 16;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();               // every warp is through with its ring
+    float (*o_s)[G][kAttnMaxD] = reinterpret_cast<float (*)[G][kAttnMaxD]>(attn_smem);
+    static_assert(S * 8 * kAttnMaxD * 4 <= kAttnSmemBytes, "the sums take the rings' place");
+    __shared__ float m_s[S][8], l_s[S][8];
+    const int st = 2 * warp + half;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        *reinterpret_cast<ulonglong2*>(&o_s[st][g][8 * sl]) = make_ulonglong2(o2[g][0], o2[g][1]);
+        *reinterpret_cast<ulonglong2*>(&o_s[st][g][8 * sl + 4]) = make_ulonglong2(o2[g][2], o2[g][3]);
+    }
+    if ((sl & 1) == 0) { m_s[st][sl >> 1] = m; l_s[st][sl >> 1] = l; }
+    __syncthreads();
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        float mx = m_s[0][g];
+#pragma unroll
+        for (int k = 1; k < S; ++k) mx = fmaxf(mx, m_s[k][g]);
+        const float ref = mx == -INFINITY ? 0.f : mx;
+        float o = 0.f, ls = 0.f;
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            const float w = __expf(m_s[k][g] - ref);
+            o += w * o_s[k][g][t];
+            ls += w * l_s[k][g];
+        }
+        float* dst = part + (((int64_t)b * nq + kvh * G + g) * n_chunks + c) * (D + 2);
+        if (t < D) dst[2 + t] = o;
+        if (t == 0) { dst[0] = mx; dst[1] = ls; }
     }
 }
 
@@ -339,7 +411,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 
 __global__ void __launch_bounds__(kCombineThreads) attn_combine_kernel(const float* __restrict__ part, const int64_t* __restrict__ pos_p,
                                                                       __nv_bfloat16* __restrict__ out, int64_t ld_out,
-                                                                      int nq, int D, int max_len, int n_chunks) {
+                                                                      int nq, int D, int max_len, int n_chunks, int span) {
     extern __shared__ float w_s[];   // [n_chunks]
     __shared__ float red[32];
     __shared__ float o_s[kCombineGroups][kAttnMaxD];
@@ -348,7 +420,7 @@ __global__ void __launch_bounds__(kCombineThreads) attn_combine_kernel(const flo
     pdl_enter();
     const int64_t pos = *pos_p;
     if (pos < 0 || pos >= max_len) return;
-    const int nc = (int)(pos / kAttnChunk) + 1;
+    const int nc = (int)(pos / span) + 1;
     const float* src = part + ((int64_t)b * nq + head) * n_chunks * (D + 2);
     float mx = -INFINITY;
     for (int c = tid; c < nc; c += kCombineThreads) {
@@ -542,6 +614,13 @@ extern "C" size_t hxq_attn_decode_workspace_bytes(int32_t B, int32_t nq, int32_t
     return (size_t)B * nq * n_chunks * (D + 2) * sizeof(float);
 }
 
+// Positions per CTA: 64 while that many CTAs (for a full cache) can be resident at once or nearly, else as
+// many times 64 as keep about 16 CTAs per SM: fewer partial results to combine, and still several waves to even out.
+static int attn_span(int n_chunks, int nkv, int B) {
+    const int64_t r = (int64_t)n_chunks * nkv * B / (148 * 16);
+    return kAttnChunk * (int)(r < 1 ? 1 : (r > n_chunks ? n_chunks : r));
+}
+
 extern "C" int hxq_attn_decode(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, const int64_t* pos,
                                void* out, int64_t ld_out, void* workspace, size_t workspace_bytes, int32_t B, int32_t nq,
                                int32_t nkv, int32_t D, int32_t max_len, float scale, hxq_stream_t stream) {
@@ -553,14 +632,30 @@ extern "C" int hxq_attn_decode(const void* q, int64_t ld_q, const void* k_cache,
     if (!workspace || workspace_bytes < hxq_attn_decode_workspace_bytes(B, nq, D, max_len)) return HXQ_E_WORKSPACE;
     const int n_chunks = (max_len + kAttnChunk - 1) / kAttnChunk;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    if (launch_pdl(attn_partial_kernel, dim3(n_chunks, nkv, B), dim3(kAttnThreads), 0, s,
-                   reinterpret_cast<const __nv_bfloat16*>(q), ld_q, reinterpret_cast<const __nv_bfloat16*>(k_cache),
-                   reinterpret_cast<const __nv_bfloat16*>(v_cache), pos, reinterpret_cast<float*>(workspace), (int)nq, (int)nkv,
-                   (int)D, (int)max_len, n_chunks, scale) != cudaSuccess)
-        return HXQ_E_LAUNCH;
-    const cudaError_t e = launch_pdl(attn_combine_kernel, dim3(nq, B), dim3(kCombineThreads), n_chunks * sizeof(float), s,
-                                     reinterpret_cast<const float*>(workspace), pos, reinterpret_cast<__nv_bfloat16*>(out), ld_out,
-                                     (int)nq, (int)D, (int)max_len, n_chunks);
+    const int span = attn_span(n_chunks, nkv, B);
+    const dim3 grid((max_len + span - 1) / span, nkv, B);
+    const __nv_bfloat16 *qp = reinterpret_cast<const __nv_bfloat16*>(q), *kp = reinterpret_cast<const __nv_bfloat16*>(k_cache),
+                        *vp = reinterpret_cast<const __nv_bfloat16*>(v_cache);
+    float* ws = reinterpret_cast<float*>(workspace);
+    cudaError_t e = cudaErrorInvalidValue;
+    auto partial = [&](auto kernel) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmemBytes) != cudaSuccess) return cudaErrorInvalidValue;
+        return launch_pdl(kernel, grid, dim3(kAttnThreads), kAttnSmemBytes, s, qp, ld_q, kp, vp, pos, ws, (int)nq, (int)nkv, (int)D, (int)max_len,
+                          n_chunks, span, scale);
+    };
+    switch (nq / nkv) {
+        case 1: e = partial(attn_partial_kernel<1>); break;
+        case 2: e = partial(attn_partial_kernel<2>); break;
+        case 3: e = partial(attn_partial_kernel<3>); break;
+        case 4: e = partial(attn_partial_kernel<4>); break;
+        case 5: e = partial(attn_partial_kernel<5>); break;
+        case 6: e = partial(attn_partial_kernel<6>); break;
+        case 7: e = partial(attn_partial_kernel<7>); break;
+        default: e = partial(attn_partial_kernel<8>); break;
+    }
+    if (e != cudaSuccess) return HXQ_E_LAUNCH;
+    e = launch_pdl(attn_combine_kernel, dim3(nq, B), dim3(kCombineThreads), n_chunks * sizeof(float), s, (const float*)ws, pos,
+                   reinterpret_cast<__nv_bfloat16*>(out), ld_out, (int)nq, (int)D, (int)max_len, n_chunks, span);
     return e == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
 
