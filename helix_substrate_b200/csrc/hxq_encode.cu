@@ -1,12 +1,10 @@
-// The encoder's passes over a dense weight: order statistics, one-dimensional k-means, nearest-code
-// assignment, outlier positions and the per-group affine fit.  All of them stream the weight (4 bytes
+// The encoder's passes over a dense weight: order statistics, nearest-code assignment, outlier
+// positions and the per-group affine fit.  All of them stream the weight (4 bytes
 // a value) once per pass and do little per value: bound by memory, a weight of up to 126 MB by L2.
 //
-// The torch operators they replace spent, on a 3584 x 3584 weight, 113 ms: kthvalue works a whole
-// tensor with one thread block, k-means scattered 500 K atomic additions into 256 addresses ten times
-// over and asked the host after each, and the fit made a dozen fp64 copies of the weight.  Here the
-// whole encoder takes 0.55 ms on it: fit 84 us, k-means 53, assignment 29, the two selections 45, the
-// outlier passes 22, the sample's sort 60, the rest launches.
+// The torch operators they replace spent over 100 ms on a 3584 x 3584 weight: kthvalue works a whole
+// tensor with one thread block, and the fit made a dozen fp64 copies of the weight.  Here: the two selections 45 us, an
+// assignment 29, the outlier passes 22, the fit 48.
 
 #include "hxq_common.cuh"
 
@@ -102,84 +100,6 @@ __global__ void select_init_kernel(SelectState* st, int64_t r0, int64_t r1) {
     st->prefix[0] = st->prefix[1] = 0u;
 }
 
-// ---- k-means on a sorted sample -------------------------------------------------------------------
-// The points nearest to a centroid are a run of the sorted sample between two midpoints, so an
-// iteration is 255 binary searches and 256 differences of the sample's prefix sums: all iterations and
-// the stop test run in one block, nothing is scattered and the host is not asked.
-__device__ __forceinline__ float max_nan(float a, float b) { return (a > b || isnan(a)) ? a : b; }
-__device__ __forceinline__ bool after(float a, float b) { return a > b || (isnan(a) && !isnan(b)); }    // a sorts behind b
-
-__global__ void __launch_bounds__(256) kmeans_kernel(const float* __restrict__ s, const double* __restrict__ prefix, int n,
-                                                     int k, int iters, double rtol, float* __restrict__ out) {
-    __shared__ float c[256];
-    __shared__ int bound[256];
-    __shared__ float red[8];
-    __shared__ int out_of_order;
-    const int i = threadIdx.x;
-    if (i < k) {      // percentile start: linear interpolation between order statistics
-        const double q = k == 1 ? 0.0 : (i < k / 2 ? i * (1.0 / (k - 1)) : 1.0 - (k - 1 - i) * (1.0 / (k - 1)));
-        const double pos = q * (double)(n - 1);
-        int lo = (int)floor(pos);
-        lo = lo < 0 ? 0 : (lo > n - 1 ? n - 1 : lo);
-        const int hi = lo + 1 < n ? lo + 1 : n - 1;
-        const float frac = (float)(pos - lo);
-        c[i] = __fadd_rn(__fmul_rn(s[lo], __fsub_rn(1.f, frac)), __fmul_rn(s[hi], frac));
-    }
-    __syncthreads();
-    double range = (double)__fsub_rn(c[k - 1], c[0]);
-    if (range == 0.0) range = 1.0;
-    for (int it = 0; it < iters; ++it) {
-        if (i < k) {
-            int b = n;
-            if (i < k - 1) {      // points <= the midpoint (exact in fp64) belong to centroids 0 .. i
-                const double mid = ((double)c[i] + (double)c[i + 1]) * 0.5;
-                int lo = 0, hi = n;
-                while (lo < hi) {
-                    const int m = (lo + hi) >> 1;
-                    if ((double)s[m] <= mid) lo = m + 1; else hi = m;
-                }
-                b = lo;
-            }
-            bound[i] = b;
-        }
-        __syncthreads();
-        float moved = 0.f, mean = 0.f;
-        if (i < k) {
-            const int lo = i ? bound[i - 1] : 0, hi = bound[i];
-            mean = c[i];
-            if (hi > lo) {      // the prefix sums skip infinities and NaNs, which a sorted run has at its ends
-                const float ends = s[lo] + s[hi - 1];
-                mean = isfinite(s[lo]) && isfinite(s[hi - 1]) ? (float)((prefix[hi - 1] - (lo ? prefix[lo - 1] : 0.0)) / (double)(hi - lo)) : ends;
-            }
-            moved = fabsf(mean - c[i]);
-        }
-#pragma unroll
-        for (int off = 16; off; off >>= 1) moved = max_nan(moved, __shfl_xor_sync(0xffffffffu, moved, off));
-        if ((i & 31) == 0) red[i >> 5] = moved;
-        __syncthreads();
-        moved = red[0];
-#pragma unroll
-        for (int w = 1; w < 8; ++w) moved = max_nan(moved, red[w]);
-        if ((double)moved < rtol * range) break;      // uniform; the step that is small enough is not taken
-        if (i < k) c[i] = mean;
-        __syncthreads();
-    }
-    __syncthreads();
-    // the means of ascending runs ascend but for a last-bit tie of roundings
-    if (i == 0) out_of_order = 0;
-    __syncthreads();
-    if (i + 1 < k && after(c[i], c[i + 1])) out_of_order = 1;
-    __syncthreads();
-    if (out_of_order) {
-        for (int round = 0; round < k; ++round) {
-            const int a = 2 * i + (round & 1);
-            if (a + 1 < k && after(c[a], c[a + 1])) { const float x = c[a]; c[a] = c[a + 1]; c[a + 1] = x; }
-            __syncthreads();
-        }
-    }
-    if (i < k) out[i] = c[i];
-}
-
 // ---- nearest code ----------------------------------------------------------------------------------
 // index = number of midpoints below the value.  A midpoint of two fp32 codes is exact in fp64; the
 // largest fp32 not above it separates the same fp32 values, so the search compares fp32.  The 255
@@ -265,48 +185,68 @@ __global__ void __launch_bounds__(256) outlier_fill_kernel(const float* __restri
 }
 
 // ---- per-(row, group) least squares of w on its code's value, excluded positions left out -----------
-// A warp per group, fp64 sums; `exclude` ascends, so a group's entries are one (mostly empty) run of it.
+// Eight lanes per group, four groups per warp (a warp per group spent most of its time in the five exchange
+// steps of five fp64 sums: 84 us for 100 K groups of 128, this 48): 16 consecutive values per lane where groups
+// and addresses allow 16-byte loads, else every eighth.  fp64 sums; `exclude` ascends, so a group's
+// entries are one (mostly empty) run of it.
 __global__ void __launch_bounds__(256) fit_kernel(const float* __restrict__ w, const uint8_t* __restrict__ idx,
-                                                  const float* __restrict__ cb, int64_t n_groups, int group,
+                                                  const float* __restrict__ cb, int64_t n_groups, int group, int vec,
                                                   const int64_t* __restrict__ exclude, int64_t n_ex,
                                                   float* __restrict__ s_out, float* __restrict__ t_out) {
     __shared__ float cb_s[256];
     cb_s[threadIdx.x] = cb[threadIdx.x];
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < n_groups; g += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int lane = threadIdx.x & 31, sl = lane & 7;
+    const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 3;
+    for (int64_t g0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane) >> 3; g0 < n_groups; g0 += step) {
+        const int64_t g = g0 + (lane >> 3);
+        const bool ok = g < n_groups;           // (lanes of a missing group stay in the exchanges)
         const int64_t first = g * group;
-        int64_t e0 = 0, e1 = n_ex;
+        int64_t e0 = 0, e1 = ok ? n_ex : 0;
         while (e0 < e1) {
             const int64_t m = (e0 + e1) >> 1;
             if (exclude[m] < first) e0 = m + 1; else e1 = m;
         }
-        int64_t next = e0 < n_ex ? exclude[e0] : INT64_MAX;     // first excluded position not below this group
-        const bool any = next < first + group;
+        const bool any = ok && e0 < n_ex && exclude[e0] < first + group;
         double n = 0, sc = 0, sw = 0, scc = 0, scw = 0;
-        for (int i = lane; i < group; i += 32) {
-            const double v = w[first + i], c = cb_s[idx[first + i]];
-            bool out = false;
+        auto add = [&](float wv, uint32_t code, int i) {
             if (any) {
-                for (int64_t e = e0; e < n_ex && exclude[e] <= first + i; ++e) out = exclude[e] == first + i;
+                for (int64_t e = e0; e < n_ex && exclude[e] <= first + i; ++e)
+                    if (exclude[e] == first + i) return;
             }
-            if (!out) {
-                n += 1.0;
-                sc += c;
-                sw += v;
-                scc = __dadd_rn(scc, __dmul_rn(c, c));
-                scw = __dadd_rn(scw, __dmul_rn(c, v));
-            }
-        }
+            const double v = wv, c = cb_s[code];
+            n += 1.0;
+            sc += c;
+            sw += v;
+            scc = __dadd_rn(scc, __dmul_rn(c, c));
+            scw = __dadd_rn(scw, __dmul_rn(c, v));
+        };
+        if (ok && vec) {
+            for (int i = 16 * sl; i < group; i += 128) {
+                const uint4 q = *reinterpret_cast<const uint4*>(idx + first + i);
+                const uint32_t word[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int off = 16; off; off >>= 1) {
+                for (int j = 0; j < 4; ++j) {
+                    const float4 f = *reinterpret_cast<const float4*>(w + first + i + 4 * j);
+                    add(f.x, word[j] & 0xffu, i + 4 * j);
+                    add(f.y, (word[j] >> 8) & 0xffu, i + 4 * j + 1);
+                    add(f.z, (word[j] >> 16) & 0xffu, i + 4 * j + 2);
+                    add(f.w, word[j] >> 24, i + 4 * j + 3);
+                }
+            }
+        } else if (ok) {
+            for (int i = sl; i < group; i += 8) add(w[first + i], idx[first + i], i);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int off = 4; off; off >>= 1) {
             n += __shfl_xor_sync(0xffffffffu, n, off);
             sc += __shfl_xor_sync(0xffffffffu, sc, off);
             sw += __shfl_xor_sync(0xffffffffu, sw, off);
             scc += __shfl_xor_sync(0xffffffffu, scc, off);
             scw += __shfl_xor_sync(0xffffffffu, scw, off);
         }
-        if (lane == 0) {
+        if (ok && sl == 0) {
             // products and differences rounded one by one: a group of one code has a determinant of exactly zero
             const double den = __dsub_rn(__dmul_rn(n, scc), __dmul_rn(sc, sc));
             const double num = __dsub_rn(__dmul_rn(n, scw), __dmul_rn(sc, sw));
@@ -350,14 +290,6 @@ extern "C" int hxq_encode_select2(const float* v, int64_t n, int64_t rank0, int6
     return cudaGetLastError() == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
 
-extern "C" int hxq_encode_kmeans(const float* sorted, const double* prefix, int32_t n, int32_t k, int32_t max_iters, double rtol,
-                                 float* centroids, hxq_stream_t stream) {
-    if (!sorted || !prefix || !centroids) return HXQ_E_ARG;
-    if (n <= 0 || k <= 0 || k > 256) return HXQ_E_SHAPE;
-    hxq::enc::kmeans_kernel<<<1, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(sorted, prefix, n, k, max_iters, rtol, centroids);
-    return cudaGetLastError() == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
-}
-
 extern "C" int hxq_encode_assign(const float* w, int64_t n, const float* codebook, int32_t k, uint8_t* indices, hxq_stream_t stream) {
     if (!w || !codebook || !indices) return HXQ_E_ARG;
     if (n <= 0 || k <= 0 || k > 256) return HXQ_E_SHAPE;
@@ -384,7 +316,8 @@ extern "C" int hxq_encode_fit(const float* w, const uint8_t* indices, const floa
                               const int64_t* exclude, int64_t n_exclude, float* scales, float* offsets, hxq_stream_t stream) {
     if (!w || !indices || !codebook || !scales || !offsets || (n_exclude > 0 && !exclude)) return HXQ_E_ARG;
     if (n_groups <= 0 || group_size <= 0 || n_exclude < 0) return HXQ_E_SHAPE;
-    hxq::enc::fit_kernel<<<hxq::enc::blocks_for(n_groups * 32, 256, 148 * 16), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        w, indices, codebook, n_groups, group_size, exclude, n_exclude, scales, offsets);
+    const int vec = group_size % 16 == 0 && hxq::aligned_to(w, 16) && hxq::aligned_to(indices, 16);
+    hxq::enc::fit_kernel<<<hxq::enc::blocks_for(n_groups * 8, 256, 148 * 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        w, indices, codebook, n_groups, group_size, vec, exclude, n_exclude, scales, offsets);
     return cudaGetLastError() == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
