@@ -42,6 +42,14 @@ int run(const hxq_desc* d, const __nv_bfloat16* xb, int64_t ldxb, int32_t M, voi
         void* split_ws, size_t split_ws_bytes, int32_t* status_word, cudaStream_t stream);
 }  // namespace gemmts
 
+namespace gemmd {    // many tokens: bf16 weight rows in scratch x activations (hxq_gemm_dense.cu)
+int64_t product_cost(int32_t M, int32_t N, int32_t K, int n_sm);
+int run(const __nv_bfloat16* x, int64_t ldx, int32_t M, const __nv_bfloat16* w, int32_t N, int32_t K,
+        const float* bias, void* y, int y_dtype, int64_t ldy, int n_sm, int32_t* status_word, cudaStream_t stream);
+}  // namespace gemmd
+
+int dequant_blocked(const hxq_desc* d, int32_t row0, int32_t row1, __nv_bfloat16* out, cudaStream_t stream);   // hxq_dequant.cu
+
 namespace gemm {
 
 constexpr int BM = 128;        // output rows per CTA = UMMA M
@@ -97,9 +105,14 @@ struct GemmArgs {
     float* partial;        // [splits][M][out_features] fp32 partial products when split, else nullptr
 };
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
+// bf16x2(c0 * s + t, c1 * s + t): one packed fp32 FMA, each half rounded like fmaf.
+__device__ __forceinline__ uint32_t affine_pack(float c0, float c1, float s, float t) {
+    uint32_t r;
+    asm("{\n\t.reg .b64 c, s, t;\n\t.reg .f32 lo, hi;\n\t"
+        "mov.b64 c, {%1, %2};\n\tmov.b64 s, {%3, %3};\n\tmov.b64 t, {%4, %4};\n\t"
+        "fma.rn.f32x2 c, c, s, t;\n\tmov.b64 {lo, hi}, c;\n\t"
+        "cvt.rn.bf16x2.f32 %0, hi, lo;\n\t}" : "=r"(r) : "f"(c0), "f"(c1), "f"(s), "f"(t));
+    return r;
 }
 
 template <int BN>
@@ -350,18 +363,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_idx, const __grid_constant__
                 const float sc = sc_c[pass], of = of_c[pass];
                 const uint4 q = *reinterpret_cast<const uint4*>(idx_s + r * BK + jc * 16);
                 const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-                float v[16];
+                uint32_t v[8];      // bf16 pairs
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
+                for (int j = 0; j < 16; j += 2) {
                     // ((code << 8) | lane*8) >> 1 = code*128 + lane*4
-                    const uint32_t off = __byte_perm(w[j >> 2], lane4x2, 0x5504u | (uint32_t)((j & 3) << 4)) >> 1;
-                    v[j] = fmaf(*reinterpret_cast<const float*>(lut + off), sc, of);
+                    const uint32_t o0 = __byte_perm(w[j >> 2], lane4x2, 0x5504u | (uint32_t)((j & 3) << 4)) >> 1;
+                    const uint32_t o1 = __byte_perm(w[j >> 2], lane4x2, 0x5504u | (uint32_t)(((j + 1) & 3) << 4)) >> 1;
+                    v[j >> 1] = affine_pack(*reinterpret_cast<const float*>(lut + o0), *reinterpret_cast<const float*>(lut + o1), sc, of);
                 }
-                uint4 lo, hi;
-                lo.x = pack_bf16x2(v[0], v[1]);   lo.y = pack_bf16x2(v[2], v[3]);
-                lo.z = pack_bf16x2(v[4], v[5]);   lo.w = pack_bf16x2(v[6], v[7]);
-                hi.x = pack_bf16x2(v[8], v[9]);   hi.y = pack_bf16x2(v[10], v[11]);
-                hi.z = pack_bf16x2(v[12], v[13]); hi.w = pack_bf16x2(v[14], v[15]);
+                const uint4 lo = make_uint4(v[0], v[1], v[2], v[3]), hi = make_uint4(v[4], v[5], v[6], v[7]);
                 char* arow = st + r * 128;
                 *reinterpret_cast<uint4*>(arow + (((2 * jc) ^ (r & 7)) << 4)) = lo;
                 *reinterpret_cast<uint4*>(arow + (((2 * jc + 1) ^ (r & 7)) << 4)) = hi;
@@ -541,6 +551,54 @@ bool fast_ok(const hxq_desc* d) {
 
 static int64_t x_pad(const hxq_desc* d) { return ((int64_t)d->in_features + 7) / 8 * 8; }
 
+// ---- two passes: weight rows to bf16 scratch, then the dense product -----------------------------
+constexpr int64_t DENSE_SCRATCH = 144ll << 20;      // most bytes of one run of rows
+constexpr int64_t DENSE_IN_L2 = 72ll << 20;         // a run that stays in the 126 MB L2 between the passes
+
+static int64_t k_pad(const hxq_desc* d) { return ((int64_t)d->in_features + 63) / 64 * 64; }   // columns of a scratch row
+
+// Estimated times in units of 0.01 us, fitted to the kernels on Qwen2.5-7B projections (us, graph replay, one pass /
+// two passes):
+//                   512 tokens   640          1024         2048         8192
+//   [18944 x 3584]  76 / 101     144 / 116    146 / 139    286 / 232    1161 / 791
+//   [3584 x 18944]  96 / 135     318 / 153    319 / 156    316 / 258    1318 / 852
+//   [3584 x 3584]   39 / 36      72 / 37      72 / 39      73 / 57      284 / 160
+//   [512 x 3584]    22 / 29      68 / 30      68 / 28      72 / 32      71 / 36
+// One pass: a 128 x 512 tile takes 1.25 us per 64-column step, a 128 x 256 one 1.0, plus 6 a launch, or 10 and the fp32
+// partials' traffic when K is split.
+static int64_t one_pass_cost(const hxq_desc* d, int32_t M, int n_sm) {
+    const int BN = pick_bn(M), grid_m = (M + BN - 1) / BN, grid_o = (d->out_features + BM - 1) / BM;
+    const int steps = (d->in_features + BK - 1) / BK, splits = pick_splits(grid_m, grid_o, steps, n_sm);
+    const int64_t tiles = (int64_t)grid_m * grid_o, step = BN > 256 ? 125 : 100;
+    if (splits > 1) return (((steps + splits - 1) / splits + 7) & ~7) * step + 1000 + (int64_t)splits * M * d->out_features / 12500;
+    return (tiles + n_sm - 1) / n_sm * steps * step + 600;
+}
+// Two passes, one run of rows: 0.56 us per million weights to write them out, the dense product, 8 for the two
+// launches, and what the weights cost on their way to HBM and back when the run does not stay in L2.
+static int64_t two_pass_cost(const hxq_desc* d, int32_t M, int64_t rows, int n_sm) {
+    const int64_t bytes = rows * k_pad(d) * 2;
+    return 800 + rows * d->in_features / 17857 + gemmd::product_cost(M, (int32_t)rows, d->in_features, n_sm) +
+           (bytes > DENSE_IN_L2 ? bytes / 25000 : 0);
+}
+
+// Weight rows per run of the two-pass product; 0 when the call runs in one pass.
+static int dense_rows(const hxq_desc* d, int32_t M, int n_sm) {
+    if (M <= 128 || n_sm < 2) return 0;          // (up to 128 tokens the tensor-memory kernel streams the indices once)
+    const int64_t row_bytes = k_pad(d) * 2, out = d->out_features;
+    if (row_bytes * 256 > DENSE_SCRATCH) return 0;
+    const int most = (int)((out * row_bytes + DENSE_IN_L2 - 1) / DENSE_IN_L2) + 1;
+    int64_t best = 0, best_cost = one_pass_cost(d, M, n_sm);
+    for (int runs = (int)((out * row_bytes + DENSE_SCRATCH - 1) / DENSE_SCRATCH); runs <= most; ++runs) {    // equal runs of whole row tiles
+        int64_t r = ((out + runs - 1) / runs + 255) / 256 * 256;
+        if (r * row_bytes > DENSE_SCRATCH && r > 256) continue;
+        if (r > out) r = out;
+        const int64_t whole = out / r, rest = out - whole * r;
+        const int64_t cost = whole * two_pass_cost(d, M, r, n_sm) + (rest ? two_pass_cost(d, M, rest, n_sm) : 0);
+        if (cost < best_cost) { best_cost = cost; best = r; }
+    }
+    return (int)best;
+}
+
 static size_t xcopy_bytes(const hxq_desc* d, int32_t M) { return (((size_t)M * x_pad(d) * 2 + 255) & ~(size_t)255) + 256; }
 
 size_t workspace_bytes(const hxq_desc* d, int32_t M) {
@@ -556,6 +614,12 @@ size_t workspace_bytes(const hxq_desc* d, int32_t M) {
         split = ts > split ? ts : split;
     }
     return xcopy_bytes(d, M) + split;
+}
+
+// Scratch of the two-pass product, 0 when it does not take the call.
+size_t scratch_bytes(const hxq_desc* d, int32_t M, bool x_in_place) {
+    const int rows = fast_ok(d) ? dense_rows(d, M, sm_count()) : 0;
+    return rows ? (x_in_place ? 0 : xcopy_bytes(d, M)) + (size_t)rows * k_pad(d) * 2 : 0;
 }
 
 template <int BN>
@@ -597,6 +661,22 @@ int run(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t ldx, v
         void* sws = (workspace && ws_bytes > off) ? reinterpret_cast<char*>(workspace) + off : nullptr;
         return gemmts::run(d, reinterpret_cast<const __nv_bfloat16*>(xb), ldxb, M, y, y_dtype, ldy, sws,
                            sws ? ws_bytes - off : 0, status_word, stream);
+    }
+    if (const int rows = dense_rows(d, M, sm_count())) {
+        const size_t off = x_in_place ? 0 : xcopy_bytes(d, M);
+        if (workspace && aligned_to(workspace, 32) && ws_bytes >= off + (size_t)rows * k_pad(d) * 2) {
+            __nv_bfloat16* wb = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<char*>(workspace) + off);
+            for (int32_t r0 = 0; r0 < d->out_features; r0 += rows) {
+                const int32_t r1 = d->out_features - r0 < rows ? d->out_features : r0 + rows;
+                int st = dequant_blocked(d, r0, r1, wb, stream);
+                if (st == HXQ_OK)
+                    st = gemmd::run(reinterpret_cast<const __nv_bfloat16*>(xb), ldxb, M, wb, r1 - r0, d->in_features,
+                                    d->bias ? d->bias + r0 : nullptr, reinterpret_cast<char*>(y) + (int64_t)r0 * dtype_size(y_dtype),
+                                    y_dtype, ldy, sm_count(), status_word, stream);
+                if (st != HXQ_OK) return st;
+            }
+            return HXQ_OK;
+        }
     }
     const int BN = pick_bn(M);
     CUtensorMap mi, mx;
@@ -653,6 +733,11 @@ int run(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t ldx, v
 extern "C" size_t hxq_gemm_workspace_bytes(const hxq_desc* d, int32_t M) {
     if (hxq::validate_desc(d) != HXQ_OK || M <= 0) return 0;
     return hxq::gemm::workspace_bytes(d, M);
+}
+
+extern "C" size_t hxq_gemm_scratch_bytes(const hxq_desc* d, int32_t M, int x_in_place) {
+    if (hxq::validate_desc(d) != HXQ_OK || M <= 0) return 0;
+    return hxq::gemm::scratch_bytes(d, M, x_in_place != 0);
 }
 
 extern "C" int hxq_gemm(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t ldx, void* y,

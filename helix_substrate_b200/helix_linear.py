@@ -98,7 +98,7 @@ class HelixLinear(nn.Module):
         self._cuda_graph_mode = False
         # "fused" (default) and "naive": the fused sm_100a kernels.  "buffered": the reference's default mode
         # (helix_linear.py:556-634) - the whole weight dequantised into a shared 16-bit buffer by hxq_dequant,
-        # then one dense library GEMM; worth choosing for prefill beyond ~1000 tokens.
+        # then one dense library GEMM.  (From a few hundred tokens on the fused mode runs in two passes itself.)
         self._forward_mode = "fused"
         self._weight_buffer = None
         self._wave_enabled = False

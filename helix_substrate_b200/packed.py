@@ -15,6 +15,7 @@ from ._lib import HxqDesc, HXQ_F32, HXQ_F16, HXQ_BF16
 _DT = {torch.float32: HXQ_F32, torch.float16: HXQ_F16, torch.bfloat16: HXQ_BF16}
 
 GEMV_MAX_M = 16      # most tokens hxq_gemv takes per call
+GEMM_TS_MAX_M = 128  # most tokens of the tensor-memory kernel; beyond, hxq_gemm may run in two passes
 GEMV_MAX_M_16BIT = 4  # bf16 / fp16 activations: beyond four tokens the tensor-memory kernel is faster
 
 
@@ -158,8 +159,7 @@ class HxqWeight:
                     _lib.check(st, "hxq_gemv")
                     m0 += mm
             else:
-                nb = L.hxq_gemm_workspace_bytes(C.byref(self.desc), M)
-                ws = _workspace(self.device, nb, "gemm")
+                ws = self._gemm_scratch(x, xd)
                 sw = _status_word(self.device)
                 st = L.hxq_gemm(C.byref(self.desc), C.c_void_p(x.data_ptr()), xd, M, x.stride(0),
                                 C.c_void_p(out.data_ptr()), _dt(out.dtype), out.stride(0),
@@ -167,6 +167,21 @@ class HxqWeight:
                                 0 if ws is None else ws.numel(), C.c_void_p(sw.data_ptr()), stream)
                 _lib.check(st, "hxq_gemm")
         return out
+
+    def _gemm_scratch(self, x: torch.Tensor, xd: int) -> Optional[torch.Tensor]:
+        """Scratch of one hxq_gemm call.  The two-pass product's (bf16 weight rows, tens of MB) comes from
+        the caching allocator for this call alone: nothing large is kept per stream, and a capture draws
+        it from its graph's pool.  Short of memory the call runs in one pass, on the kept workspace."""
+        L, M = _lib.lib(), x.shape[0]
+        if M > GEMM_TS_MAX_M:
+            in_place = xd == HXQ_BF16 and x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0
+            nb = L.hxq_gemm_scratch_bytes(C.byref(self.desc), M, in_place)
+            if nb:
+                try:
+                    return torch.empty(nb, dtype=torch.uint8, device=self.device)
+                except torch.OutOfMemoryError:
+                    pass
+        return _workspace(self.device, L.hxq_gemm_workspace_bytes(C.byref(self.desc), M), "gemm")
 
     # ---- dense rows ----------------------------------------------------------
     def dequant(self, row0: int = 0, row1: Optional[int] = None,

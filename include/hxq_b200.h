@@ -184,6 +184,11 @@ int hxq_gemv_packed6(const uint8_t* packed, int32_t out_features, int32_t in_fea
  * clears the part of the workspace they need first.
  */
 size_t hxq_gemm_workspace_bytes(const hxq_desc* d, int32_t M);
+/* From a few hundred tokens on a run of weight rows is better written out once as bf16 and multiplied by a
+ * dense kernel than dequantised again for every token tile.  hxq_gemm does that whenever the workspace has
+ * room for it: this many bytes (0: the call gains nothing from more than hxq_gemm_workspace_bytes), at most
+ * 144 MB on top of the bf16 copy of x.  x_in_place: x is bf16 with 16-byte aligned rows, so no copy is made. */
+size_t hxq_gemm_scratch_bytes(const hxq_desc* d, int32_t M, int x_in_place);
 int hxq_gemm(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t ldx,
              void* y, int y_dtype, int64_t ldy,
              void* workspace, size_t workspace_bytes, int32_t* status_word,
