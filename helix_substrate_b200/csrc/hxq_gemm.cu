@@ -526,12 +526,13 @@ void launch_splitk_reduce(const float* partial, int splits, int M, int out_featu
 // K slices per output tile: enough CTAs to fill the GPU when the tile grid alone does not
 // (one token tile x few row tiles, e.g. down_proj at M <= 64), at least four K steps each.
 static int pick_bn(int M) { return M > 256 ? 512 : (M > 128 ? 256 : (M > 64 ? 128 : 64)); }
-static int sm_count() {
+static int sm_count() {      // asked once per device
+    static int cached[64] = {0};
     int n_sm = 148, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        n_sm <= 0)
-        n_sm = 148;
-    return n_sm;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return n_sm;
+    if (cached[dev] == 0)
+        cached[dev] = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n_sm > 0 ? n_sm : 148;
+    return cached[dev];
 }
 static int pick_splits(int grid_m, int grid_o, int k_steps, int n_sm) {
     // only with a single token tile: with more, the fp32 partials (splits x M x OUT) cost more traffic than

@@ -524,12 +524,13 @@ namespace gemmts {
 
 // ---- host side ---------------------------------------------------------------------
 
-static int sm_count() {
+static int sm_count() {      // asked once per device
+    static int cached[64] = {0};
     int n_sm = 148, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        n_sm <= 0)
-        n_sm = 148;
-    return n_sm;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return n_sm;
+    if (cached[dev] == 0)
+        cached[dev] = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n_sm > 0 ? n_sm : 148;
+    return cached[dev];
 }
 
 static int pick_bn(int M) { return M > 64 ? 128 : (M > 32 ? 64 : (M > 16 ? 32 : 16)); }

@@ -258,7 +258,7 @@ class HelixLinear(nn.Module):
     def packed(self, with_sidecar: bool = True) -> HxqWeight:
         """The descriptor over this module's CUDA buffers (built on first use,
         dropped whenever buffers move or reload)."""
-        if not self.indices.is_cuda:
+        if not self._buffers["indices"].is_cuda:
             raise RuntimeError(
                 "HelixLinear runs on CUDA only: move the module and its input to a B200 "
                 "(.cuda()); there is no CPU forward path. No silent fallback.")
@@ -294,21 +294,22 @@ class HelixLinear(nn.Module):
         if getattr(self, "_forward_mode", "fused") == "buffered":
             self._last_dispatch_path = "buffered"
             return self._forward_buffered(x)
-        self._last_dispatch_path = "fused"
+        self.__dict__["_last_dispatch_path"] = "fused"      # plain attributes: Module.__setattr__ costs as much as a launch
         return self._run(x, x.dtype if x.dtype in (torch.float16, torch.bfloat16, torch.float32) else torch.float32)
 
     def _run(self, x: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
         shape = x.shape
-        x2 = x.reshape(-1, self.in_features)
+        flat = x.ndim == 2 and shape[1] == self.in_features
+        x2 = x if flat else x.reshape(-1, self.in_features)
         if x2.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             x2 = x2.float()
         if self.has_channel_scales:  # AWQ: weights live in scaled space (helix_linear.py:478-480)
             x2 = x2 / self.channel_scales.to(x2.dtype).unsqueeze(0)
-        apply_sc = self._policy_decide(x2) if self._csr_rowptr is not None else False
+        apply_sc = self._policy_decide(x2) if self._buffers.get("_csr_rowptr") is not None else False
         w = self.packed(with_sidecar=apply_sc)
         svd = self.has_svd and not self._cell_skip_svd
         y = w.matmul(x2, out_dtype=torch.float32 if svd else out_dtype)
-        self._last_dispatch = {
+        self.__dict__["_last_dispatch"] = {
             "dispatch_selected": "hxq_gemv_sm100a" if uses_gemv(x2.shape[0], x2.dtype) else "hxq_gemm_sm100a",
             "tokens": int(x2.shape[0]), "vq_dim": 1,
         }
@@ -316,7 +317,7 @@ class HelixLinear(nn.Module):
             xf = x2.float()
             y += ((xf @ self.svd_Vt.t()) * self.svd_s.unsqueeze(0)) @ self.svd_U.t()
             y = y.to(out_dtype)
-        return y.reshape(*shape[:-1], self.out_features)
+        return y if flat else y.reshape(*shape[:-1], self.out_features)
 
     # the reference's per-path entry points all land on the same kernels
     def _forward_fused(self, x: torch.Tensor) -> torch.Tensor:

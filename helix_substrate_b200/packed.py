@@ -37,14 +37,14 @@ _workspaces: dict = {}
 _status_words: dict = {}
 
 
-def _workspace(device: torch.device, nbytes: int, kind: str = "gemv") -> Optional[torch.Tensor]:
+def _workspace(device: torch.device, nbytes: int, kind: str = "gemv", stream: Optional[int] = None) -> Optional[torch.Tensor]:
     """Scratch, one per (device, stream, kernel family); grown on demand.
     hxq_gemv needs its workspace zeroed and leaves it zeroed, so it is cleared
     only when (re)allocated; hxq_gemm uses its own as plain scratch (a bf16 copy
     of the activations) and leaves it dirty - the two are never shared."""
     if nbytes == 0:
         return None
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, kind)
+    key = (device.index, torch.cuda.current_stream(device).cuda_stream if stream is None else stream, kind)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         if torch.cuda.is_current_stream_capturing():
@@ -113,6 +113,9 @@ class HxqWeight:
         for t in (codebook, rowptr, cols, deltas, values, self.bias, scales, offsets):
             assert t is None or t.device == self.device, "all buffers of one weight live on one device"
         self.desc = self._fill()
+        self._dref = C.byref(self.desc)
+        self._gemv_bytes: dict = {}     # tokens per call (1 .. 16) -> scratch bytes of hxq_gemv
+        self._gemm_bytes: dict = {}     # tokens (1 .. GEMM_TS_MAX_M) -> workspace bytes of hxq_gemm
 
     def _fill(self) -> HxqDesc:
         p = lambda t: None if t is None else C.c_void_p(t.data_ptr())
@@ -142,46 +145,58 @@ class HxqWeight:
             out = torch.empty(M, self.out_features, device=self.device, dtype=out_dtype)
         if M == 0:
             return out
-        L = _lib.lib()
-        stream = C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
         use_gemv = uses_gemv(M, x.dtype) if force is None else (force == "gemv")
-        with torch.cuda.device(self.device):
-            if use_gemv:
-                y, m0 = out, 0
-                while m0 < M:  # hxq_gemv takes at most 16 tokens per call
-                    mm = min(GEMV_MAX_M, M - m0)
-                    nb = L.hxq_gemv_workspace_bytes(C.byref(self.desc), mm)
-                    ws = _workspace(self.device, nb)
-                    st = L.hxq_gemv(C.byref(self.desc), C.c_void_p(x[m0:].data_ptr()), xd, mm, x.stride(0),
-                                    C.c_void_p(y[m0:].data_ptr()), _dt(out.dtype), out.stride(0),
-                                    None if ws is None else C.c_void_p(ws.data_ptr()),
-                                    0 if ws is None else ws.numel(), stream)
-                    _lib.check(st, "hxq_gemv")
-                    m0 += mm
-            else:
-                ws = self._gemm_scratch(x, xd)
-                sw = _status_word(self.device)
-                st = L.hxq_gemm(C.byref(self.desc), C.c_void_p(x.data_ptr()), xd, M, x.stride(0),
-                                C.c_void_p(out.data_ptr()), _dt(out.dtype), out.stride(0),
-                                None if ws is None else C.c_void_p(ws.data_ptr()),
-                                0 if ws is None else ws.numel(), C.c_void_p(sw.data_ptr()), stream)
-                _lib.check(st, "hxq_gemm")
+        if torch.cuda.current_device() == self.device.index:
+            self._launch(x, xd, M, out, use_gemv)
+        else:
+            with torch.cuda.device(self.device):
+                self._launch(x, xd, M, out, use_gemv)
         return out
 
-    def _gemm_scratch(self, x: torch.Tensor, xd: int) -> Optional[torch.Tensor]:
+    def _launch(self, x: torch.Tensor, xd: int, M: int, out: torch.Tensor, use_gemv: bool) -> None:
+        """The launches of one product on the current stream of the weight's device, which is current.
+        At a few tokens the kernel is shorter than this function: raw integers instead of ctypes and
+        stream objects, and the scratch size (a function of the descriptor and M) asked for once."""
+        L = _lib.lib()
+        dev = self.device.index
+        stream = torch._C._cuda_getCurrentRawStream(dev)
+        xp, yp, ldx, ldy, yd = x.data_ptr(), out.data_ptr(), x.stride(0), out.stride(0), _dt(out.dtype)
+        if use_gemv:
+            xs, ys = x.element_size(), out.element_size()
+            m0 = 0
+            while m0 < M:  # hxq_gemv takes at most 16 tokens per call
+                mm = min(GEMV_MAX_M, M - m0)
+                nb = self._gemv_bytes.get(mm)
+                if nb is None:
+                    nb = self._gemv_bytes[mm] = L.hxq_gemv_workspace_bytes(self._dref, mm)
+                ws = _workspace(self.device, nb, "gemv", stream)
+                st = L.hxq_gemv(self._dref, xp + m0 * ldx * xs, xd, mm, ldx, yp + m0 * ldy * ys, yd, ldy,
+                                None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(), stream)
+                _lib.check(st, "hxq_gemv")
+                m0 += mm
+        else:
+            ws = self._gemm_scratch(L, x, xd, M, stream)
+            st = L.hxq_gemm(self._dref, xp, xd, M, ldx, yp, yd, ldy, None if ws is None else ws.data_ptr(),
+                            0 if ws is None else ws.numel(), _status_word(self.device).data_ptr(), stream)
+            _lib.check(st, "hxq_gemm")
+
+    def _gemm_scratch(self, L, x: torch.Tensor, xd: int, M: int, stream: int) -> Optional[torch.Tensor]:
         """Scratch of one hxq_gemm call.  The two-pass product's (bf16 weight rows, tens of MB) comes from
         the caching allocator for this call alone: nothing large is kept per stream, and a capture draws
         it from its graph's pool.  Short of memory the call runs in one pass, on the kept workspace."""
-        L, M = _lib.lib(), x.shape[0]
-        if M > GEMM_TS_MAX_M:
-            in_place = xd == HXQ_BF16 and x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0
-            nb = L.hxq_gemm_scratch_bytes(C.byref(self.desc), M, in_place)
-            if nb:
-                try:
-                    return torch.empty(nb, dtype=torch.uint8, device=self.device)
-                except torch.OutOfMemoryError:
-                    pass
-        return _workspace(self.device, L.hxq_gemm_workspace_bytes(C.byref(self.desc), M), "gemm")
+        if M <= GEMM_TS_MAX_M:
+            nb = self._gemm_bytes.get(M)
+            if nb is None:
+                nb = self._gemm_bytes[M] = L.hxq_gemm_workspace_bytes(self._dref, M)
+            return _workspace(self.device, nb, "gemm", stream)
+        in_place = xd == HXQ_BF16 and x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0
+        nb = L.hxq_gemm_scratch_bytes(self._dref, M, in_place)
+        if nb:
+            try:
+                return torch.empty(nb, dtype=torch.uint8, device=self.device)
+            except torch.OutOfMemoryError:
+                pass
+        return _workspace(self.device, L.hxq_gemm_workspace_bytes(self._dref, M), "gemm", stream)
 
     # ---- dense rows ----------------------------------------------------------
     def dequant(self, row0: int = 0, row1: Optional[int] = None,
