@@ -487,12 +487,14 @@ __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gate, const __nv
 // the shared-memory pipe, not HBM, the limit from two tokens on); fp32 accumulation, one warp
 // reduction per row.  W is long-lived (see the weight precondition of the compressed products): its
 // first loads are issued before the wait for the previous kernel.
-template <int MP>
+//
+// R rows and U pieces per step, R * U = 8 loads in flight either way: four rows of two pieces, or, when the matrix
+// has too few groups of four rows to go round, two rows of four: twice the warps, and half the steps in each.
+template <int MP, int R, int U>
 __global__ void __launch_bounds__(256) dense_gemv_kernel(const __nv_bfloat16* __restrict__ W, int64_t ldw, int n_out, int n_in,
                                                          const __nv_bfloat16* __restrict__ x, int64_t ldx, void* y, int y_dtype,
                                                          int64_t ldy, int M) {
     extern __shared__ __align__(16) float xs[];          // [MP][n_in]
-    constexpr int R = 4, U = 2;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int n_chunk = n_in >> 3;
@@ -515,10 +517,18 @@ __global__ void __launch_bounds__(256) dense_gemv_kernel(const __nv_bfloat16* __
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (grp < n_groups) load_w(grp, 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int i = threadIdx.x; i < MP * n_in; i += blockDim.x) {
-        const int m = i / n_in, k = i - m * n_in;
-        xs[i] = m < M ? __bfloat162float(x[(int64_t)m * ldx + k]) : 0.f;
-    }
+#pragma unroll
+    for (int m = 0; m < MP; ++m)
+        if (m < M && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0) {      // eight at a time
+            for (int c = threadIdx.x; c < n_chunk; c += blockDim.x) {
+                float f[8];
+                unpack8(*reinterpret_cast<const uint4*>(x + (int64_t)m * ldx + c * 8), f);
+                *reinterpret_cast<float4*>(xs + m * n_in + c * 8) = make_float4(f[0], f[1], f[2], f[3]);
+                *reinterpret_cast<float4*>(xs + m * n_in + c * 8 + 4) = make_float4(f[4], f[5], f[6], f[7]);
+            }
+        } else {
+            for (int k = threadIdx.x; k < n_in; k += blockDim.x) xs[m * n_in + k] = m < M ? __bfloat162float(x[(int64_t)m * ldx + k]) : 0.f;
+        }
     __syncthreads();
     for (; grp < n_groups; grp += groups_total) {
         float acc[R][MP];
@@ -669,15 +679,16 @@ extern "C" int hxq_swiglu(const void* gate, const void* up, void* out, int32_t B
     return e == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
 
-template <int MP>
-static int launch_dense_gemv(const __nv_bfloat16* W, int64_t ldw, int n_out, int n_in, const __nv_bfloat16* x, int64_t ldx,
-                             void* y, int y_dtype, int64_t ldy, int M, cudaStream_t stream) {
+template <int MP, int R, int U>
+static int launch_dense_gemv_as(const __nv_bfloat16* W, int64_t ldw, int n_out, int n_in, const __nv_bfloat16* x, int64_t ldx,
+                             void* y, int y_dtype, int64_t ldy, int M, cudaStream_t stream,
+                                bool only_if_busy) {
     const size_t smem = (size_t)MP * n_in * sizeof(float);
     static size_t smem_set[64] = {0};
     int dev = 0, n_sm = 148, occ = 1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return HXQ_E_DEVICE;
     if (smem > 48 * 1024 && smem_set[dev] < smem) {
-        if (cudaFuncSetAttribute(dense_gemv_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(dense_gemv_kernel<MP, R, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return HXQ_E_SHAPE;
         smem_set[dev] = smem;
     }
@@ -689,16 +700,23 @@ static int launch_dense_gemv(const __nv_bfloat16* W, int64_t ldw, int n_out, int
         sm_cached[dev] = n_sm;
     }
     if (occ_cached[dev] == 0 || occ_smem[dev] != smem) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dense_gemv_kernel<MP>, 256, smem) != cudaSuccess || occ < 1) occ = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dense_gemv_kernel<MP, R, U>, 256, smem) != cudaSuccess || occ < 1) occ = 1;
         occ_cached[dev] = occ;
         occ_smem[dev] = smem;
     }
     int grid = sm_cached[dev] * occ_cached[dev];
-    const int need = (n_out + 31) / 32;      // eight warps of four rows per CTA
+    const int need = (n_out + 8 * R - 1) / (8 * R);      // eight warps of R rows per CTA
+    if (only_if_busy && need < grid) return 1;           // too few groups of rows for the resident warps
     if (grid > need) grid = need;
-    const cudaError_t e = launch_pdl(dense_gemv_kernel<MP>, dim3(grid), dim3(256), smem, stream, W, ldw, n_out, n_in, x, ldx, y,
+    const cudaError_t e = launch_pdl(dense_gemv_kernel<MP, R, U>, dim3(grid), dim3(256), smem, stream, W, ldw, n_out, n_in, x, ldx, y,
                                      y_dtype, ldy, M);
     return e == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
+}
+template <int MP>
+static int launch_dense_gemv(const __nv_bfloat16* W, int64_t ldw, int n_out, int n_in, const __nv_bfloat16* x, int64_t ldx,
+                             void* y, int y_dtype, int64_t ldy, int M, cudaStream_t stream) {
+    const int st = launch_dense_gemv_as<MP, 4, 2>(W, ldw, n_out, n_in, x, ldx, y, y_dtype, ldy, M, stream, true);
+    return st <= 0 ? st : launch_dense_gemv_as<MP, 2, 4>(W, ldw, n_out, n_in, x, ldx, y, y_dtype, ldy, M, stream, false);
 }
 
 extern "C" int hxq_dense_gemv(const void* weight, int32_t out_features, int32_t in_features, int64_t ldw, const void* x,
