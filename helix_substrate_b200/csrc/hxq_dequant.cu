@@ -241,14 +241,18 @@ static int launch_vec_stm(const DequantArgs& a, cudaStream_t stream) {
     }
     const int vec_per_row = a.k_pad >> 4;
     const int rows = a.row1 - a.row0;
-    const int per_unit = vec_per_row >= 128 ? 1 : 128 / vec_per_row;
-    const int segs = vec_per_row >= 128 ? (vec_per_row + kUnitPieces - 1) / kUnitPieces : 1;
+    // pieces per unit: 256, fewer (in whole warps) when the matrix would not go round the resident warps twice - a
+    // 512 x 3584 one in units of a row ran on 32 SMs
+    const int64_t share = (int64_t)rows * vec_per_row / (148 * 2 * (kVecThreads / 32) * 2) / 32 * 32;
+    const int pieces = share < 32 ? 32 : (share > kUnitPieces ? kUnitPieces : (int)share);
+    const int per_unit = vec_per_row * 2 > pieces ? 1 : pieces / vec_per_row;
+    const int segs = per_unit > 1 ? 1 : (vec_per_row + pieces - 1) / pieces;
     const int64_t blocks64 = ((int64_t)((rows + per_unit - 1) / per_unit) * segs + kVecThreads / 32 - 1) / (kVecThreads / 32);
     const int blocks = (int)(blocks64 < 148 * 2 ? blocks64 : 148 * 2);
     int shift = -1;
     if (a.group_size > 0 && (a.group_size & (a.group_size - 1)) == 0)
         for (shift = 0; (1 << shift) < a.group_size; ) ++shift;
-    // v / vec_per_row as a multiplication, for units of several rows: v < 128 (exact while v * vec_per_row < 2^32)
+    // v / vec_per_row as a multiplication, for units of several rows: v < 256 (exact while v * vec_per_row < 2^32)
     const uint32_t magic = vec_per_row > 1 ? (uint32_t)(((1ull << 32) + vec_per_row - 1) / vec_per_row) : 0u;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
