@@ -503,24 +503,66 @@ __global__ void __launch_bounds__(256) to_bf16_kernel(const void* x, int x_dtype
 }
 
 // y[m, o] = sum over the K slices of partial[z][m][o], + bias, rounded once (fixed order: deterministic).
+// One row of blocks per token, four outputs per thread where alignment allows (VEC): a launch of a few MB whose
+// time is its latency, so it is launched dependent and waits on the device for the product's partials.
+template <bool VEC>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, int splits, int M, int out_features,
                                                             const float* __restrict__ bias, void* y, int y_dtype, int64_t ldy) {
+    constexpr int W = VEC ? 4 : 1;
     const int64_t total = (int64_t)M * out_features;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int m = (int)(i / out_features), o = (int)(i - (int64_t)m * out_features);
-        float v = 0.f;
-        for (int z = 0; z < splits; ++z) v += partial[(int64_t)z * total + i];
-        if (bias != nullptr) v += bias[o];
-        store_from_f32(y, (int64_t)m * ldy + o, v, y_dtype);
+    const int o = (blockIdx.x * 256 + threadIdx.x) * W;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (o >= out_features) return;
+    for (int m = blockIdx.y; m < M; m += gridDim.y) {
+        const float* p = partial + (int64_t)m * out_features + o;
+        float v[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) v[e] = 0.f;
+        for (int z = 0; z < splits; ++z) {
+            if constexpr (VEC) {
+                const float4 q = *reinterpret_cast<const float4*>(p + (int64_t)z * total);
+                v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
+            } else {
+                v[0] += p[(int64_t)z * total];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e)
+            if (bias != nullptr) v[e] += bias[o + e];
+        const int64_t at = (int64_t)m * ldy + o;
+        if constexpr (VEC) {
+            if (y_dtype == HXQ_F32) {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + at) = make_float4(v[0], v[1], v[2], v[3]);
+            } else if (y_dtype == HXQ_BF16) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(y) + at) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            } else {
+                const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(y) + at) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
+        } else {
+            store_from_f32(y, at, v[0], y_dtype);
+        }
     }
 }
 
 void launch_splitk_reduce(const float* partial, int splits, int M, int out_features, const float* bias, void* y,
                           int y_dtype, int64_t ldy, cudaStream_t stream) {
-    const int64_t total = (int64_t)M * out_features;
-    int blocks = (int)((total + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(partial, splits, M, out_features, bias, y, y_dtype, ldy);
+    const bool vec = out_features % 4 == 0 && aligned_to(partial, 16) && aligned_to(y, 16) && ldy % 4 == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((out_features + (vec ? 1023 : 255)) / (vec ? 1024 : 256), M < 4096 ? M : 4096);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (vec) cudaLaunchKernelEx(&cfg, splitk_reduce_kernel<true>, partial, splits, M, out_features, bias, y, y_dtype, ldy);
+    else cudaLaunchKernelEx(&cfg, splitk_reduce_kernel<false>, partial, splits, M, out_features, bias, y, y_dtype, ldy);
 }
 
 // K slices per output tile: enough CTAs to fill the GPU when the tile grid alone does not

@@ -41,7 +41,7 @@
 //   gate [18944 x 3584]           28.9 / 39.5 29.3 / 39.4 30.1 / 39.4 32.0 / 46.9
 //   down [3584 x 18944], K split  40.5 / 47.9 40.3 / 48.0 41.7 / 48.6 44.2 / 58.8
 //   q [3584 x 3584], K split      15.8 / 18.6 16.1 / 19.1 18.0 / 19.7 20.3 / 24.5
-// Bound by the instruction stream of the lookups (about 6 instructions per weight) at 44 % issue.
+// Bound by the instruction stream: 8 warp instructions per 32 weights at 54 % issue.
 //
 // Every mbarrier wait is clock-bounded; a wait that gives up raises a CTA-wide abort flag and the
 // global status word (HXQ_E_TIMEOUT); every other wait of the CTA then returns at its next poll,
