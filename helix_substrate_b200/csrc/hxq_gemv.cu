@@ -81,6 +81,7 @@ struct GemvArgs {
 struct GemvPlan {
     int nch, nrb, kbase, grid, warps_per_cta, units, max_parts, rbl_max;
     size_t counter_bytes, scratch_bytes;
+    bool dependent = true;     // set-up may overlap the previous kernel's tail
 };
 
 template <int MP>
@@ -1216,10 +1217,10 @@ static cudaLaunchConfig_t gemv_launch_config(const GemvPlan& p, int smem_bytes, 
     cfg.blockDim = dim3(p.warps_per_cta * 32);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set-up may overlap the previous kernel's tail
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_weights_on_stream ? 0 : 1;   // weights still being written on this stream: no early start
+    cfg.numAttrs = p.dependent ? 1 : 0;
     return cfg;
 }
 
@@ -1336,6 +1337,9 @@ int gemv_any_m(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t
             const int wedge = (MP == 4) ? GemvCfg<4>::kEdgeMaxWarps : (MP == 2 ? GemvCfg<2>::kEdgeMaxWarps : GemvCfg<1>::kEdgeMaxWarps);
             if (pl.warps_per_cta > wedge) pl.warps_per_cta = wedge;
         }
+        // weights still being written on this stream: no early start - but for the launches after the call's first,
+        // which started when they were complete
+        pl.dependent = m0 > 0 || !g_weights_on_stream;
         int st;
         if (MP == 1) st = launch_fast<1>(a, pl, lean ? &tmap : nullptr, stream);
         else if (MP == 2) st = launch_fast<2>(a, pl, lean ? &tmap : nullptr, stream);
