@@ -119,11 +119,6 @@ def lib() -> C.CDLL:
     L.hxq_encode_select_workspace_bytes.argtypes = []
     L.hxq_encode_select2.restype = C.c_int
     L.hxq_encode_select2.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
-    L.hxq_encode_kmeans_workspace_bytes.restype = C.c_size_t
-    L.hxq_encode_kmeans_workspace_bytes.argtypes = []
-    L.hxq_encode_kmeans.restype = C.c_int
-    L.hxq_encode_kmeans.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_double, C.c_void_p, C.c_void_p, C.c_size_t,
-                                    C.c_void_p]
     L.hxq_encode_assign.restype = C.c_int
     L.hxq_encode_assign.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]
     L.hxq_encode_outlier_runs.restype = C.c_int64

@@ -1,11 +1,10 @@
-// The encoder's passes over a dense weight: order statistics, one-dimensional k-means, nearest-code
-// assignment, outlier positions and the per-group affine fit.  All of them stream the weight (4 bytes
+// The encoder's passes over a dense weight: order statistics, nearest-code assignment, outlier
+// positions and the per-group affine fit.  All of them stream the weight (4 bytes
 // a value) once per pass and do little per value: bound by memory, a weight of up to 126 MB by L2.
 //
 // The torch operators they replace spent over 100 ms on a 3584 x 3584 weight: kthvalue works a whole
-// tensor with one thread block, k-means scattered 500 K atomic additions into 256 addresses ten times
-// over and asked the host after each, and the fit made a dozen fp64 copies of the weight.  Here: the two selections 45 us, an
-// assignment 29, the outlier passes 22, the fit 48, k-means 240; 0.61 ms with the sample's sort and the host.
+// tensor with one thread block, and the fit made a dozen fp64 copies of the weight.  Here: the two selections 45 us, an
+// assignment 29, the outlier passes 22, the fit 48.
 
 #include "hxq_common.cuh"
 
@@ -99,102 +98,6 @@ __global__ void __launch_bounds__(1024) select_pick_kernel(const unsigned int* _
 __global__ void select_init_kernel(SelectState* st, int64_t r0, int64_t r1) {
     st->rank[0] = r0; st->rank[1] = r1;
     st->prefix[0] = st->prefix[1] = 0u;
-}
-
-// ---- k-means on a sorted sample -------------------------------------------------------------------
-// The points nearest to a centroid are a run of the sorted sample between two midpoints.  A warp per centroid
-// finds its run by two binary searches and adds it up as ONE chain of fp32 additions in sample order -
-// what the scattered fp32 additions it replaces came to, to within their order, so codebooks stay what they
-// were (sums in more precision move every midpoint by the chain's rounding bias, and codes with it).  The
-// stop test is made on the device: ten steps are twenty small launches, and the host is not asked.
-struct KmeansState {
-    double range;
-    int moved;        // largest movement of a step, as ordered bits of a non-negative float (a NaN is above all)
-    int done;
-};
-constexpr int KM_WARPS = 8;
-
-__device__ __forceinline__ int run_end(const float* __restrict__ s, int n, const float* c, int k, int i) {   // first point behind centroid i's
-    if (i >= k - 1) return n;
-    const double mid = ((double)c[i] + (double)c[i + 1]) * 0.5;       // exact; points on it belong to the lower centroid
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int m = (lo + hi) >> 1;
-        if ((double)s[m] <= mid) lo = m + 1; else hi = m;
-    }
-    return lo;
-}
-
-__global__ void __launch_bounds__(256) kmeans_init_kernel(const float* __restrict__ s, int n, int k, float* c, KmeansState* st) {
-    const int i = threadIdx.x;
-    if (i < k) {      // percentile start: linear interpolation between order statistics
-        const double q = k == 1 ? 0.0 : (i < k / 2 ? i * (1.0 / (k - 1)) : 1.0 - (k - 1 - i) * (1.0 / (k - 1)));
-        const double pos = q * (double)(n - 1);
-        int lo = (int)floor(pos);
-        lo = lo < 0 ? 0 : (lo > n - 1 ? n - 1 : lo);
-        const int hi = lo + 1 < n ? lo + 1 : n - 1;
-        const float frac = (float)(pos - lo);
-        c[i] = __fadd_rn(__fmul_rn(s[lo], __fsub_rn(1.f, frac)), __fmul_rn(s[hi], frac));
-    }
-    __syncthreads();
-    if (i == 0) {
-        const double range = (double)__fsub_rn(c[k - 1], c[0]);
-        st->range = range == 0.0 ? 1.0 : range;
-        st->moved = 0;
-        st->done = 0;
-    }
-}
-
-__global__ void __launch_bounds__(32 * KM_WARPS) kmeans_step_kernel(const float* __restrict__ s, int n, int k, const float* __restrict__ c,
-                                                                    float* __restrict__ next, KmeansState* st) {
-    const int i = blockIdx.x * KM_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= k || st->done) return;
-    const int lo = i ? run_end(s, n, c, k, i - 1) : 0, hi = run_end(s, n, c, k, i);
-    float sum = 0.f;
-    float v = lo + lane < hi ? s[lo + lane] : 0.f;
-    for (int b = lo; b < hi; b += 32) {
-        const float w = b + 32 + lane < hi ? s[b + 32 + lane] : 0.f;      // the next 32 are on their way
-        const int cnt = hi - b < 32 ? hi - b : 32;
-        if (cnt == 32) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, v, j));
-        } else {
-            for (int j = 0; j < cnt; ++j) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, v, j));
-        }
-        v = w;
-    }
-    const float mean = hi > lo ? __fdiv_rn(sum, (float)(hi - lo)) : c[i];
-    if (lane == 0) {
-        next[i] = mean;
-        const float moved = fabsf(__fsub_rn(mean, c[i]));
-        atomicMax(&st->moved, isnan(moved) ? 0x7fffffff : __float_as_int(moved));
-    }
-}
-
-// Takes the step unless it was small enough to stop; the last call leaves the centroids ascending (the means of
-// ascending runs ascend but for a last-bit tie of roundings).
-__device__ __forceinline__ bool after(float a, float b) { return a > b || (isnan(a) && !isnan(b)); }    // a sorts behind b
-
-__global__ void __launch_bounds__(256) kmeans_take_kernel(int k, double rtol, float* c, const float* __restrict__ next, KmeansState* st, int step, int last) {
-    const int i = threadIdx.x;
-    __shared__ int out_of_order;
-    const bool done = st->done != 0;
-    const int bits = st->moved;
-    const bool stop = done || (bits != 0x7fffffff && (double)__int_as_float(bits) < rtol * st->range);
-    __syncthreads();
-    if (step && !stop && i < k) c[i] = next[i];
-    if (i == 0) { st->done = stop; st->moved = 0; out_of_order = 0; }
-    if (!last) return;
-    __syncthreads();
-    if (i + 1 < k && after(c[i], c[i + 1])) out_of_order = 1;
-    __syncthreads();
-    if (out_of_order) {
-        for (int round = 0; round < k; ++round) {
-            const int a = 2 * i + (round & 1);
-            if (a + 1 < k && after(c[a], c[a + 1])) { const float x = c[a]; c[a] = c[a + 1]; c[a + 1] = x; }
-            __syncthreads();
-        }
-    }
 }
 
 // ---- nearest code ----------------------------------------------------------------------------------
@@ -384,27 +287,6 @@ extern "C" int hxq_encode_select2(const float* v, int64_t n, int64_t rank0, int6
     select_pick_kernel<1><<<1, 1024, 0, stream>>>(hist + BINS, st, out);
     select_count_kernel<2><<<blocks, 512, 0, stream>>>(v, n, st, hist + 3 * BINS);
     select_pick_kernel<2><<<1, 1024, 0, stream>>>(hist + 3 * BINS, st, out);
-    return cudaGetLastError() == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
-}
-
-extern "C" size_t hxq_encode_kmeans_workspace_bytes(void) { return sizeof(hxq::enc::KmeansState) + 256 * sizeof(float); }
-
-extern "C" int hxq_encode_kmeans(const float* sorted, int32_t n, int32_t k, int32_t max_iters, double rtol, float* centroids,
-                                 void* workspace, size_t workspace_bytes, hxq_stream_t stream_) {
-    using namespace hxq::enc;
-    if (!sorted || !centroids) return HXQ_E_ARG;
-    if (n <= 0 || k <= 0 || k > 256) return HXQ_E_SHAPE;
-    if (!workspace || workspace_bytes < hxq_encode_kmeans_workspace_bytes()) return HXQ_E_WORKSPACE;
-    if (!hxq::aligned_to(workspace, 8)) return HXQ_E_ALIGN;
-    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    KmeansState* st = reinterpret_cast<KmeansState*>(workspace);
-    float* next = reinterpret_cast<float*>(st + 1);
-    kmeans_init_kernel<<<1, 256, 0, stream>>>(sorted, n, k, centroids, st);
-    for (int it = 0; it < max_iters; ++it) {
-        kmeans_step_kernel<<<(k + KM_WARPS - 1) / KM_WARPS, 32 * KM_WARPS, 0, stream>>>(sorted, n, k, centroids, next, st);
-        kmeans_take_kernel<<<1, 256, 0, stream>>>(k, rtol, centroids, next, st, 1, it == max_iters - 1);
-    }
-    if (max_iters <= 0) kmeans_take_kernel<<<1, 256, 0, stream>>>(k, rtol, centroids, next, st, 0, 1);
     return cudaGetLastError() == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
 

@@ -72,18 +72,6 @@ def _subsample_positions_on(n: int, device: torch.device) -> torch.Tensor:
     return pos
 
 
-def _kmeans_on_gpu(sample: torch.Tensor, n_clusters: int, max_iters: int, rtol: float) -> torch.Tensor:
-    """The same iteration on a sorted fp32 sample: runs between midpoints, each summed in sample order."""
-    L = _lib.lib()
-    cents = torch.empty(n_clusters, dtype=torch.float32, device=sample.device)
-    ws = torch.empty(L.hxq_encode_kmeans_workspace_bytes(), dtype=torch.uint8, device=sample.device)
-    with torch.cuda.device(sample.device):
-        st = L.hxq_encode_kmeans(_ptr(sample), sample.numel(), n_clusters, max_iters, rtol, _ptr(cents), _ptr(ws), ws.numel(),
-                                 _stream(sample.device))
-    _lib.check(st, "hxq_encode_kmeans")
-    return cents
-
-
 def kmeans_codebook(flat: torch.Tensor, n_clusters: int = 256, max_iters: int = 10,
                     rtol: float = 1e-3) -> torch.Tensor:
     """1-D Lloyd on the reference's RandomState(42) subsample with percentile
@@ -97,8 +85,6 @@ def kmeans_codebook(flat: torch.Tensor, n_clusters: int = 256, max_iters: int = 
     else:
         sample = flat
     sample = sample.float().sort().values
-    if flat.is_cuda and flat.ndim == 1 and n > 0 and 1 <= n_clusters <= 256:
-        return _kmeans_on_gpu(sample, n_clusters, max_iters, rtol)
     q = torch.linspace(0, 1, n_clusters, device=flat.device, dtype=torch.float64)
     pos = q * (sample.numel() - 1)
     lo = pos.floor().long()
@@ -106,10 +92,15 @@ def kmeans_codebook(flat: torch.Tensor, n_clusters: int = 256, max_iters: int = 
     frac = (pos - lo).float()
     cents = sample[lo] * (1 - frac) + sample[hi] * frac
     rng = float(cents[-1] - cents[0]) or 1.0
+    codes = torch.arange(n_clusters, device=flat.device) if flat.is_cuda and n_clusters <= 256 else None
     for _ in range(max_iters):
         assign = assign_indices(sample, cents).long()
+        # fp32 additions, scattered: on a GPU their order is the hardware's, and with it a codebook's last bits.
         sums = torch.zeros(n_clusters, device=flat.device).index_add_(0, assign, sample)
-        cnts = torch.zeros(n_clusters, device=flat.device).index_add_(0, assign, torch.ones_like(sample))
+        if codes is not None:     # the codes of a sorted sample ascend: a cluster's size is the distance of their places
+            cnts = torch.diff(torch.searchsorted(assign, codes, right=True), prepend=codes.new_zeros(1)).float()
+        else:
+            cnts = torch.zeros(n_clusters, device=flat.device).index_add_(0, assign, torch.ones_like(sample))
         new = torch.where(cnts > 0, sums / cnts.clamp(min=1), cents)
         moved = float((new - cents).abs().max())
         if moved < rtol * rng:

@@ -289,12 +289,6 @@ int hxq_allreduce_add_rmsnorm(void* const* peer_buffers, void* const* peer_flags
 size_t hxq_encode_select_workspace_bytes(void);
 int hxq_encode_select2(const float* v, int64_t n, int64_t rank0, int64_t rank1, float* out, void* workspace,
                        size_t workspace_bytes, hxq_stream_t stream);
-/* k <= 256 centroids of an ascending sample: percentile start, at most max_iters Lloyd steps, stop before the first
- * step that moves no centroid by rtol of the start's range; sums in fp32, one addition after the other in
- * sample order.  workspace: hxq_encode_kmeans_workspace_bytes() of 8-byte aligned scratch. */
-size_t hxq_encode_kmeans_workspace_bytes(void);
-int hxq_encode_kmeans(const float* sorted, int32_t n, int32_t k, int32_t max_iters, double rtol, float* centroids,
-                      void* workspace, size_t workspace_bytes, hxq_stream_t stream);
 /* indices[i] = number of midpoints of the ascending codebook (k <= 256) that lie below w[i]: the nearest entry,
  * the lower one at a tie. */
 int hxq_encode_assign(const float* w, int64_t n, const float* codebook, int32_t k, uint8_t* indices, hxq_stream_t stream);

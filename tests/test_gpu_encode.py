@@ -60,25 +60,35 @@ def test_assignment_is_exact_at_midpoints(k, n):
 
 @pytest.mark.parametrize("n,k", [(1, 1), (3, 8), (5000, 16), (200_000, 256), (600_000, 256)])
 def test_kmeans_matches_the_cpu_path(n, k):
-    """Same start, steps and stop; fp32 sums of n / k values of size up to 5, in sample order on both sides but
-    for how the CPU splits them: at most (n / k) * 2^-24 of a mean apart each step, ten steps."""
+    """Same start, steps and stop, counts from the sorted sample; fp32 sums of n / k values of size up to 5 in
+    another order differ by at most (n / k) * 2^-24 of a mean each step, ten steps."""
     from helix_substrate_b200.hxq_writer_gpu import kmeans_codebook
     v = torch.randn(n, generator=torch.Generator().manual_seed(n))
     a, b = kmeans_codebook(v.to(DEV), k).cpu(), kmeans_codebook(v, k)
     assert a.shape == b.shape and torch.equal(a, a.sort().values)
     assert float((a - b).abs().max()) <= 10 * 5 * max(1, n // k) * 2.0 ** -24
-    assert torch.equal(a, kmeans_codebook(v.to(DEV), k).cpu()), "bit-identical from run to run"
     assert torch.equal(kmeans_codebook(torch.full((100,), 0.5, device=DEV), 4).cpu(), torch.full((4,), 0.5))
 
 
-def test_kmeans_of_an_infinite_sample():
-    """An infinity reaches its own centroid only, as in the CPU path; no steps: the percentile start."""
+def test_kmeans_roundings_do_not_line_up():
+    """One cluster of half a million values: its fp32 sum reaches 2^20, where an addition rounds by up to 1/16.  Added
+    in ascending order the roundings of neighbours agree (the mean is off by 2.5e-4); scattered ones mostly cancel
+    (5e-5 to 8e-5 in four runs, the square root of their number times 1/28 being 2e-5)."""
     from helix_substrate_b200.hxq_writer_gpu import kmeans_codebook
-    v = torch.cat([torch.tensor([float("-inf")]), torch.arange(1000.0)])
-    a, b = kmeans_codebook(v.to(DEV), 8, max_iters=3).cpu(), kmeans_codebook(v, 8, max_iters=3)
-    assert torch.equal(a.isfinite(), b.isfinite())
-    v = torch.randn(1000)
-    assert torch.equal(kmeans_codebook(v.to(DEV), 8, max_iters=0).cpu(), kmeans_codebook(v, 8, max_iters=0))
+    v = 1 + 3 * torch.rand(500_000, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1))
+    mean = float(v.double().mean())
+    assert abs(float(kmeans_codebook(v, 1, max_iters=1, rtol=0.0)) - mean) < 1.5e-4 * mean
+
+
+@pytest.mark.parametrize("special", [float("-inf"), float("inf"), float("nan")])
+def test_kmeans_of_a_special_value(special):
+    """An infinity or a NaN reaches the same centroids as in the CPU path, and the others move as there; no steps:
+    the percentile start."""
+    from helix_substrate_b200.hxq_writer_gpu import kmeans_codebook
+    v = torch.cat([torch.tensor([special]), torch.arange(1000.0)])
+    for iters in (0, 1, 3):
+        a, b = kmeans_codebook(v.to(DEV), 8, max_iters=iters).cpu(), kmeans_codebook(v, 8, max_iters=iters)
+        torch.testing.assert_close(a, b, rtol=1e-6, atol=1e-6, equal_nan=True)
 
 
 @pytest.mark.parametrize("n_out,n_in,G", [(1, 1, 1), (3, 96, 32), (5, 300, 100), (64, 1024, 128)])
