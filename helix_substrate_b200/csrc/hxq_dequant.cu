@@ -87,7 +87,9 @@ template <int OUT_DT, int STM, bool BLK>
 __global__ void __launch_bounds__(kVecThreads, 2)
 dequant_vec_kernel(const DequantArgs a, const int rows_per_unit, const int segs, const int group_shift, const uint32_t div_magic) {
     extern __shared__ __align__(256) char lut[];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // Only the two-pass product lets the next kernel in early: its product waits.  What follows hxq_dequant may take
+    // `out` for a long-lived weight and read it before its own wait.
+    if constexpr (BLK) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     {
         constexpr int PER = 256 / (kVecThreads / 32);
@@ -97,7 +99,7 @@ dequant_vec_kernel(const DequantArgs a, const int rows_per_unit, const int segs,
 #pragma unroll
         for (int j = 0; j < PER; ++j) *reinterpret_cast<float*>(lut + (warp * PER + j) * 256 + lane * 4) = c[j];
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // (the out buffer may still be read by the kernel before this one)
+    if constexpr (BLK) asm volatile("griddepcontrol.wait;" ::: "memory");      // (the scratch may still be read by the product before this one)
     __syncthreads();
     const uint32_t lane4 = (uint32_t)lane << 2;
     const uint32_t vec_per_row = (uint32_t)a.k_pad >> 4;

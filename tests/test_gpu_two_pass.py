@@ -36,6 +36,24 @@ def test_dequant_runs_of_rows(n_out, n_in, G, st):
     assert torch.equal(wide[:, :n_in].cpu(), ref.to(torch.bfloat16)) and bool((wide[:, n_in:] == 7.0).all())
 
 
+def test_dequant_then_dense_product_on_one_stream():
+    """hxq_dequant lets nothing start before it is done: a kernel that fetches its weights ahead (the dense
+    product) finds the rows written, and not what the buffer held before."""
+    from helix_substrate_b200 import decode_ops
+    rng = np.random.default_rng(5)
+    n_out, n_in = 18944, 3584
+    cb, idx, pos, vals, _, s, t = _make(rng, n_out, n_in, 128, 0.001, bias=False)
+    w = _weight(cb, idx, pos, vals, None, s, t, 128)
+    x = torch.randn(1, n_in, device=DEV).bfloat16()
+    dense = w.dequant(dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    want = decode_ops.dense_gemv(dense, x)
+    for _ in range(5):
+        dense.fill_(7.0)
+        w.dequant(dtype=torch.bfloat16, out=dense)
+        assert torch.equal(decode_ops.dense_gemv(dense, x), want)
+
+
 def _check(M, n_out, n_in, G, xdt, ydt, bias=True, x=None, seed=0):
     rng = np.random.default_rng(M * 7 + n_out + n_in + seed)
     cb, idx, pos, vals, b, s, t = _make(rng, n_out, n_in, G, 0.001, bias=bias)
