@@ -134,8 +134,8 @@ def lib() -> C.CDLL:
 
 class weights_on_stream:
     """``with weights_on_stream():`` around a product whose descriptor buffers (codebook, indices,
-    scales, sidecar) were produced by kernels still in flight on the current stream: the decode
-    kernels then start only after those kernels have finished (see include/hxq_b200.h)."""
+    scales, sidecar; a dense product's weight) were produced by kernels still in flight on the current
+    stream: its kernels then start only after those have finished (see include/hxq_b200.h)."""
 
     def __enter__(self):
         lib().hxq_set_weights_on_stream(1)

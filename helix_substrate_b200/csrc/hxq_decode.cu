@@ -31,7 +31,7 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+static cudaError_t launch(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -41,8 +41,12 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), Args&&... args) {
+    return launch(true, kernel, std::forward<Args>(args)...);
 }
 
 __device__ __forceinline__ float block_sum(float v, float* red) {   // blockDim.x <= 1024, all threads call
@@ -708,8 +712,8 @@ static int launch_dense_gemv_as(const __nv_bfloat16* W, int64_t ldw, int n_out, 
     const int need = (n_out + 8 * R - 1) / (8 * R);      // eight warps of R rows per CTA
     if (only_if_busy && need < grid) return 1;           // too few groups of rows for the resident warps
     if (grid > need) grid = need;
-    const cudaError_t e = launch_pdl(dense_gemv_kernel<MP, R, U>, dim3(grid), dim3(256), smem, stream, W, ldw, n_out, n_in, x, ldx, y,
-                                     y_dtype, ldy, M);
+    const cudaError_t e = launch(!hxq::g_weights_on_stream, dense_gemv_kernel<MP, R, U>, dim3(grid), dim3(256), smem, stream, W, ldw, n_out,
+                                 n_in, x, ldx, y, y_dtype, ldy, M);
     return e == cudaSuccess ? HXQ_OK : HXQ_E_LAUNCH;
 }
 template <int MP>

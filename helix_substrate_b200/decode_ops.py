@@ -93,7 +93,8 @@ def dense_gemv(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None =
     """y = x @ weight.t() for a dense bf16 weight [OUT, IN] and up to four bf16 tokens (lm_head at
     decode time; the reference runs it as _BF16Linear, helix_substrate/basin_runtime.py:181-205).
     ``weight`` is a long-lived one: its first rows are fetched while the kernel in front of this one on the
-    stream still runs, so it must have been complete before that kernel started."""
+    stream still runs, so it must have been complete before that kernel started (else: inside
+    ``_lib.weights_on_stream()``)."""
     _bf16_rows(weight, "weight"); _bf16_rows(x, "x")
     M, n_in = x.shape
     n_out = weight.shape[0]

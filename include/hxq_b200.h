@@ -77,14 +77,16 @@ typedef struct hxq_desc {
 int hxq_version(void);
 
 /*
- * hxq_gemv / hxq_gemv_static start their set-up (codebook table, first index rows, scale / offset /
- * row-pointer reads) BEFORE the kernels in front of them on the stream have finished (programmatic
- * dependent launch) and only wait for those kernels before they touch x, y and the workspace.
- * PRECONDITION: every buffer named in the hxq_desc is complete before the call is enqueued - which
- * is the case for weights loaded once.  A caller that produces a descriptor's buffers with kernels
- * on the SAME stream right before the product (a codebook computed per call, indices unpacked per
- * call) brackets the call with hxq_set_weights_on_stream(1) ... (0): while set (per host thread),
- * the products launch as ordinary stream-ordered kernels.  No counterpart in the reference.
+ * hxq_gemv, hxq_gemv_static, hxq_gemm (up to 128 tokens, and its two-pass product beyond) and
+ * hxq_dense_gemv start their set-up (codebook table, first index bytes or weight rows, scale / offset /
+ * row-pointer / sidecar reads) BEFORE the kernels in front of them on the stream have finished
+ * (programmatic dependent launch) and only wait for those kernels before they touch x, y and the workspace.
+ * PRECONDITION: every buffer named in the hxq_desc (for hxq_dense_gemv the weight) is complete before the
+ * call is enqueued - which is the case for weights loaded once.  A caller that produces these buffers with
+ * kernels on the SAME stream right before the product (a codebook computed per call, indices unpacked per
+ * call, rows that hxq_dequant writes) brackets the call with hxq_set_weights_on_stream(1) ... (0): while
+ * set (per host thread), the products launch as ordinary stream-ordered kernels.  No counterpart in the
+ * reference.
  */
 void hxq_set_weights_on_stream(int on);
 
@@ -236,7 +238,8 @@ int hxq_swiglu(const void* gate, const void* up, void* out, int32_t B, int32_t n
  * (helix_substrate/tensor_policy.py:199-208) and runs as its _BF16Linear
  * (helix_substrate/basin_runtime.py:181-205).  in_features % 8 == 0 and <= 12288, ldw % 8 == 0,
  * weight 16-byte aligned; y fp32, fp16 or bf16; fp32 accumulation.  The weight must be complete
- * before the previous kernel on the stream started (it is fetched while that kernel drains). */
+ * before the previous kernel on the stream started (it is fetched while that kernel drains), unless
+ * hxq_set_weights_on_stream is on. */
 int hxq_dense_gemv(const void* weight, int32_t out_features, int32_t in_features, int64_t ldw, const void* x,
                    int32_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, hxq_stream_t stream);
 
