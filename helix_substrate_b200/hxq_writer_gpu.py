@@ -165,12 +165,19 @@ def find_outliers_percentile(weight: torch.Tensor, percentile: float):
 
 
 def _fit_on_gpu(weight: torch.Tensor, codebook: torch.Tensor, indices: torch.Tensor, group_size: int,
-                exclude: Optional[torch.Tensor], ascending: bool = False):
+                exclude: Optional[torch.Tensor], trusted: bool = False):
+    """``trusted``: ``exclude`` ascends and lies inside the matrix, and every index inside the codebook."""
     n_out, n_in = weight.shape
     w, cb, idx = weight.float().contiguous(), codebook.float(), indices.contiguous()
     cb = torch.cat([cb, cb[-1:].expand(256 - cb.numel())]) if cb.numel() < 256 else cb.contiguous()
     n_ex = 0 if exclude is None else exclude.numel()
-    if n_ex and not ascending:
+    if not trusted and not torch.cuda.is_current_stream_capturing():     # what indexing refuses: the kernel would pass over it
+        if codebook.numel() < 256 and int(idx.max()) >= codebook.numel():
+            raise IndexError(f"index {int(idx.max())} is out of bounds for a codebook of {codebook.numel()} entries")
+        lo, hi = torch.stack(exclude.aminmax()).tolist() if n_ex else (0, 0)
+        if lo < -w.numel() or hi >= w.numel():
+            raise IndexError(f"excluded position {lo if lo < -w.numel() else hi} is out of bounds for {w.numel()} weights")
+    if n_ex and not trusted:
         exclude = torch.where(exclude < 0, exclude + w.numel(), exclude).sort().values
     s = torch.empty(n_out, n_in // group_size, dtype=torch.float32, device=w.device)
     t = torch.empty_like(s)
@@ -235,8 +242,8 @@ def compress_weight(weight: torch.Tensor, n_clusters: int = 256, percentile: flo
         out["sidecar_values"] = vals.half().float()
     if group_size > 0:
         assert w.shape[1] % group_size == 0
-        # (the sidecar's positions ascend already)
-        s, t = _fit_on_gpu(w, cb, idx, group_size, pos, ascending=True) if w.is_cuda and w.numel() else fit_group_affine(w, cb, idx, group_size, pos)
+        # (the sidecar's positions and the codes are this function's own)
+        s, t = _fit_on_gpu(w, cb, idx, group_size, pos, trusted=True) if w.is_cuda and w.numel() else fit_group_affine(w, cb, idx, group_size, pos)
         out["group_scales"], out["group_offsets"] = s.to(st_dtype), t.to(st_dtype)
         out["group_size"] = group_size
     return out

@@ -111,6 +111,23 @@ def test_group_fit_matches_the_torch_path(n_out, n_in, G, n_ex):
     torch.testing.assert_close(gt.cpu(), t, rtol=1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("bad", [64, -65, 1 << 40])
+def test_group_fit_refuses_what_lies_outside(bad):
+    """An excluded position outside the matrix, a code outside the codebook: refused on both devices, the ends of
+    the range taken."""
+    from helix_substrate_b200.hxq_writer_gpu import fit_group_affine
+    w, cb, idx = torch.randn(4, 16), torch.arange(8.0), torch.arange(64).view(4, 16).remainder(8).to(torch.uint8)
+    for dev in ("cpu", DEV):
+        a = [t.to(dev) for t in (w, cb, idx)]
+        with pytest.raises(IndexError):
+            fit_group_affine(*a, 16, torch.tensor([3, bad], device=dev))
+        with pytest.raises(IndexError):
+            fit_group_affine(a[0], a[1][:7], a[2], 16)
+    ex = torch.tensor([-64, 63, -1])
+    for x, y in zip(fit_group_affine(w.to(DEV), cb.to(DEV), idx.to(DEV), 16, ex.to(DEV)), fit_group_affine(w, cb, idx, 16, ex)):
+        torch.testing.assert_close(x.cpu(), y, rtol=1e-6, atol=1e-6)
+
+
 def test_compress_weight_round_trip():
     """The whole encoder on both devices: same outliers, codes that agree but for values next to a
     midpoint, the same reconstruction error."""
