@@ -209,10 +209,11 @@ __global__ void __launch_bounds__(256) fit_kernel(const float* __restrict__ w, c
         }
         const bool any = ok && e0 < n_ex && exclude[e0] < first + group;
         double n = 0, sc = 0, sw = 0, scc = 0, scw = 0;
+        int64_t e = e0;       // this lane's place among the group's entries: its own positions ascend too
         auto add = [&](float wv, uint32_t code, int i) {
             if (any) {
-                for (int64_t e = e0; e < n_ex && exclude[e] <= first + i; ++e)
-                    if (exclude[e] == first + i) return;
+                while (e < n_ex && exclude[e] < first + i) ++e;
+                if (e < n_ex && exclude[e] == first + i) return;
             }
             const double v = wv, c = cb_s[code];
             n += 1.0;

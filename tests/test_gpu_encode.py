@@ -111,6 +111,22 @@ def test_group_fit_matches_the_torch_path(n_out, n_in, G, n_ex):
     torch.testing.assert_close(gt.cpu(), t, rtol=1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("n_in,G", [(512, 256), (600, 200), (4096, 4096)])
+@pytest.mark.parametrize("keep", [2, 3, 17])
+def test_group_fit_with_most_positions_excluded(n_in, G, keep):
+    """Lanes that skip runs of excluded positions, some of them given twice; a whole row in one group."""
+    from helix_substrate_b200.hxq_writer_gpu import fit_group_affine
+    g = torch.Generator().manual_seed(n_in + keep)
+    w, cb = torch.randn(3, n_in, generator=g), torch.randn(256, generator=g).sort().values
+    idx = torch.randint(0, 256, (3, n_in), generator=g).to(torch.uint8)
+    ex = torch.arange(3 * n_in)
+    ex = torch.cat([ex[ex % keep != 0], ex[1:7]])
+    s, t = fit_group_affine(w, cb, idx, G, ex)
+    gs, gt = fit_group_affine(w.to(DEV), cb.to(DEV), idx.to(DEV), G, ex.to(DEV))
+    torch.testing.assert_close(gs.cpu(), s, rtol=1e-6, atol=1e-6)
+    torch.testing.assert_close(gt.cpu(), t, rtol=1e-6, atol=1e-6)
+
+
 @pytest.mark.parametrize("bad", [64, -65, 1 << 40])
 def test_group_fit_refuses_what_lies_outside(bad):
     """An excluded position outside the matrix, a code outside the codebook: refused on both devices, the ends of
