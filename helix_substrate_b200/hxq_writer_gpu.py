@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from typing import Optional
 
 import torch
@@ -30,6 +31,7 @@ _KMEANS_MAX_SAMPLES = 500_000
 _subsample_cache: dict = {}
 _subsample_on_device: dict = {}     # (n, device) -> the same positions, for the sizes in use: at most _SUBSAMPLE_KEEP
 _SUBSAMPLE_KEEP = 8                 # tables of 4 MB
+_subsample_lock = threading.Lock()
 
 
 def _ptr(t: torch.Tensor) -> C.c_void_p:
@@ -58,16 +60,23 @@ def _subsample_positions(n: int) -> torch.Tensor:
     return pos
 
 
+def _keep(store: dict, key, table, most: int):
+    """``table`` in a store that all threads share, or the one another thread put there first; the oldest leave."""
+    with _subsample_lock:
+        table = store.setdefault(key, table)
+        while len(store) > most:
+            del store[next(iter(store))]
+    return table
+
+
 def _subsample_positions_on(n: int, device: torch.device) -> torch.Tensor:
     """``_subsample_positions`` on a device, kept for the few sizes a model's tensors have: the copy
     of 500 000 positions from pageable memory took longer than the k-means it feeds."""
     key = (n, device.index if device.index is not None else torch.cuda.current_device())
     pos = _subsample_on_device.get(key)
     if pos is None:
-        pos = _subsample_positions(n).to(device)          # complete on return: a copy from pageable memory
-        while len(_subsample_on_device) >= _SUBSAMPLE_KEEP:
-            _subsample_on_device.pop(next(iter(_subsample_on_device)), None)
-        _subsample_on_device[key] = pos
+        # complete on return: a copy from pageable memory
+        pos = _keep(_subsample_on_device, key, _subsample_positions(n).to(device), _SUBSAMPLE_KEEP)
     pos.record_stream(torch.cuda.current_stream(device))  # a table that is dropped outlives its use on this stream
     return pos
 

@@ -300,3 +300,32 @@ def test_six_bit_packing_round_trip_and_bit_layout():
     ref = np.stack([b0 & 63, ((b0 >> 6) | (b1 << 2)) & 63, ((b1 >> 4) | (b2 << 4)) & 63, (b2 >> 2) & 63], -1)
     assert np.array_equal(ref.reshape(7, 24), idx.numpy())
 
+
+
+def test_kept_tables_under_threads():
+    """Threads that fill one bounded store at once: nothing raised, every caller gets a table of its own key, the
+    bound holds.  (Taking the first key of a dict while another thread inserts raises.)"""
+    import sys
+    import threading
+    from helix_substrate_b200.hxq_writer_gpu import _keep
+    store, wrong = {}, []
+
+    def fill(seed):
+        try:
+            for i in range(4000):
+                key = (i * 7 + seed) % 23
+                if _keep(store, key, [key], 3) != [key]:
+                    wrong.append(key)
+        except Exception as e:      # noqa: BLE001
+            wrong.append(e)
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=fill, args=(s,)) for s in range(8)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert not wrong and 0 < len(store) <= 3
