@@ -80,6 +80,8 @@ def lib() -> C.CDLL:
     L.hxq_gemm_workspace_bytes.argtypes = [P, C.c_int32]
     L.hxq_gemm_scratch_bytes.restype = C.c_size_t
     L.hxq_gemm_scratch_bytes.argtypes = [P, C.c_int32, C.c_int]
+    L.hxq_gemm_row_tile.restype = C.c_int32
+    L.hxq_gemm_row_tile.argtypes = [P, C.c_int32, C.POINTER(C.c_int32)]
     L.hxq_gemm.restype = C.c_int
     L.hxq_gemm.argtypes = [P, C.c_void_p, C.c_int, C.c_int32, C.c_int64, C.c_void_p, C.c_int, C.c_int64,
                            C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]
@@ -92,6 +94,8 @@ def lib() -> C.CDLL:
     L.hxq_rope_append.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                   C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                   C.c_void_p]
+    L.hxq_attn_decode_span.restype = C.c_int32
+    L.hxq_attn_decode_span.argtypes = [C.c_int32, C.c_int32, C.c_int32]
     L.hxq_attn_decode_workspace_bytes.restype = C.c_size_t
     L.hxq_attn_decode_workspace_bytes.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_int32]
     L.hxq_attn_decode.restype = C.c_int

@@ -630,9 +630,17 @@ extern "C" size_t hxq_attn_decode_workspace_bytes(int32_t B, int32_t nq, int32_t
 
 // Positions per CTA: 64 while that many CTAs (for a full cache) can be resident at once or nearly, else as
 // many times 64 as keep about 16 CTAs per SM: fewer partial results to combine, and still several waves to even out.
+// The cache's length decides, not the position, so a short context in a long cache runs on few CTAs: 300 of 32768 rows at
+// batch 8 take 18 us in spans of 384 where spans of 64 would take 12, 6000 of 524288 at batch 1 34 where 14.  (A CTA per
+// 64 rows of the cache, most of them empty, took 27 and 40.)
 static int attn_span(int n_chunks, int nkv, int B) {
     const int64_t r = (int64_t)n_chunks * nkv * B / (148 * 16);
     return kAttnChunk * (int)(r < 1 ? 1 : (r > n_chunks ? n_chunks : r));
+}
+
+extern "C" int32_t hxq_attn_decode_span(int32_t B, int32_t nkv, int32_t max_len) {
+    if (B <= 0 || nkv <= 0 || max_len <= 0) return 0;
+    return attn_span((max_len + kAttnChunk - 1) / kAttnChunk, nkv, B);
 }
 
 extern "C" int hxq_attn_decode(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, const int64_t* pos,

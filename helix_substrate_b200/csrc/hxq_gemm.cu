@@ -35,7 +35,7 @@ int gemv_any_m(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t
                int64_t ldy, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 size_t gemv_workspace_bytes(const hxq_desc* d, int32_t M);
 
-namespace gemmts {   // 17 .. 128 tokens: A operand through tensor memory (hxq_gemm_ts.cu)
+namespace gemmts {   // up to 128 tokens: A operand through tensor memory (hxq_gemm_ts.cu)
 bool covers(const hxq_desc* d, int32_t M);
 size_t split_bytes(const hxq_desc* d, int32_t M);
 int run(const hxq_desc* d, const __nv_bfloat16* xb, int64_t ldxb, int32_t M, void* y, int y_dtype, int64_t ldy,
@@ -44,6 +44,7 @@ int run(const hxq_desc* d, const __nv_bfloat16* xb, int64_t ldxb, int32_t M, voi
 
 namespace gemmd {    // many tokens: bf16 weight rows in scratch x activations (hxq_gemm_dense.cu)
 int64_t product_cost(int32_t M, int32_t N, int32_t K, int n_sm);
+int32_t row_tile(int32_t M, int32_t N, int n_sm);
 int run(const __nv_bfloat16* x, int64_t ldx, int32_t M, const __nv_bfloat16* w, int32_t N, int32_t K,
         const float* bias, void* y, int y_dtype, int64_t ldy, int n_sm, int32_t* status_word, cudaStream_t stream);
 }  // namespace gemmd
@@ -781,6 +782,14 @@ extern "C" size_t hxq_gemm_workspace_bytes(const hxq_desc* d, int32_t M) {
 extern "C" size_t hxq_gemm_scratch_bytes(const hxq_desc* d, int32_t M, int x_in_place) {
     if (hxq::validate_desc(d) != HXQ_OK || M <= 0) return 0;
     return hxq::gemm::scratch_bytes(d, M, x_in_place != 0);
+}
+
+extern "C" int32_t hxq_gemm_row_tile(const hxq_desc* d, int32_t M, int32_t* rows_per_run) {
+    using namespace hxq;
+    if (validate_desc(d) != HXQ_OK || M <= 0) return 0;
+    const int rows = gemm::fast_ok(d) ? gemm::dense_rows(d, M, gemm::sm_count()) : 0;
+    if (rows_per_run) *rows_per_run = rows;
+    return rows ? gemmd::row_tile(M, rows, gemm::sm_count()) : 0;
 }
 
 extern "C" int hxq_gemm(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t ldx, void* y,

@@ -4,7 +4,8 @@
 //
 //   y[m, o] = sum_k x[m, k] * W[o, k] + bias[o]        (bf16 operands, fp32 accumulator in TMEM)
 //
-// Bound by the tensor cores.  A pair of CTAs (one TPC) owns a 256-token x BN-row tile, cta_group::2:
+// Bound by the staging of its operands (measured below).  A pair of CTAs (one TPC) owns a 256-token x
+// BN-row tile, cta_group::2:
 //
 //   * the weight rows come blocked, [K / 64][rows][64]: a stage's box is one contiguous piece (as 128-byte
 //     rows 2 K bytes apart a box took several microseconds from HBM, and a product with few token
@@ -23,7 +24,8 @@
 //
 // Measured: 1.46 PFLOP/s on [18944 x 3584] at 2048 and 8192 tokens (0.43 us per 64-column step of a pair's
 // 256 x 256 tile).  It follows the 32 KB that each SM stages per
-// step, 11 TB/s over the GPU, not the MMAs (0.27 us).
+// step, 11 TB/s over the GPU, not the MMAs (0.27 us) - a limit of this kernel, not of the machine: the library's
+// product reaches 1.64.
 //
 // BN is a launch argument, a multiple of 32 up to 256 (see pick_tile): an output width that leaves a
 // nearly empty last wave at 256 columns takes the width that fills it.
@@ -326,6 +328,12 @@ static int pick_tile(int tiles_m, int N, int pairs, int64_t& best_cost) {
         if (cost < best_cost) { best_cost = cost; best = bn; }
     }
     return best;
+}
+
+// Weight rows per tile of the product of M tokens and N rows.
+int32_t row_tile(int32_t M, int32_t N, int n_sm) {
+    int64_t cost;
+    return pick_tile((M + TM - 1) / TM, N, n_sm / 2, cost);
 }
 
 // Estimated time of the product of M tokens and N rows of K columns, in units of 0.01 us.

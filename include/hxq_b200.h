@@ -191,6 +191,9 @@ size_t hxq_gemm_workspace_bytes(const hxq_desc* d, int32_t M);
  * room for it: this many bytes (0: the call gains nothing from more than hxq_gemm_workspace_bytes), at most
  * 144 MB on top of the bf16 copy of x.  x_in_place: x is bf16 with 16-byte aligned rows, so no copy is made. */
 size_t hxq_gemm_scratch_bytes(const hxq_desc* d, int32_t M, int x_in_place);
+/* How the two-pass product of M tokens is cut: weight rows per tile, and (rows_per_run, may be NULL) weight rows
+ * per run of the scratch; 0 when the call runs in one pass. */
+int32_t hxq_gemm_row_tile(const hxq_desc* d, int32_t M, int32_t* rows_per_run);
 int hxq_gemm(const hxq_desc* d, const void* x, int x_dtype, int32_t M, int64_t ldx,
              void* y, int y_dtype, int64_t ldy,
              void* workspace, size_t workspace_bytes, int32_t* status_word,
@@ -228,6 +231,10 @@ size_t hxq_attn_decode_workspace_bytes(int32_t B, int32_t nq, int32_t D, int32_t
 int hxq_attn_decode(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, const int64_t* pos,
                     void* out, int64_t ld_out, void* workspace, size_t workspace_bytes, int32_t B, int32_t nq,
                     int32_t nkv, int32_t D, int32_t max_len, float scale, hxq_stream_t stream);
+
+/* Cache rows that one thread block of hxq_attn_decode walks: a multiple of 64, 64 while the blocks of a full
+ * cache are few, more as they grow.  Needs no device. */
+int32_t hxq_attn_decode_span(int32_t B, int32_t nkv, int32_t max_len);
 
 /* out[b, i] = silu(gate[b, i]) * up[b, i], i < n (the MLP between gate/up and down). */
 int hxq_swiglu(const void* gate, const void* up, void* out, int32_t B, int32_t n, int64_t ld_gate,

@@ -1,6 +1,7 @@
 """hxq_gemm at 5 .. 128 tokens: every warp group owns a quarter of a CTA's K range.  Box counts that do not
 divide by four, parts that start inside a block of scales, ragged ends, sidecar entries that meet in
-one packed pair; and single-query attention at the edges of its steps and spans."""
+one packed pair; and single-query attention at the edges of its steps, and of spans of one to four times
+64 rows."""
 
 import numpy as np
 import pytest
@@ -51,12 +52,39 @@ def test_dense_sidecar_rows():
 @pytest.mark.parametrize("D,max_len,pos", [(128, 64, 0), (128, 700, 63), (64, 700, 64), (8, 257, 256), (120, 2000, 1999)])
 @pytest.mark.parametrize("B", [1, 40])
 def test_attention_groups_and_edges(nq, nkv, D, max_len, pos, B):
-    """Every group size, part-filled steps and spans, head dimensions below 128 (idle lanes), rows past the
+    """Every group size, part-filled steps, head dimensions below 128 (idle lanes), rows past the
     position holding NaN (never read into the result); fp32 arithmetic on bf16 operands, bf16 result."""
     from helix_substrate_b200 import decode_ops
     g = torch.Generator(device=DEV).manual_seed(nq * D + pos)
     q = torch.randn(B, nq * D, device=DEV, generator=g).bfloat16()
     kc, vc = (torch.randn(B, nkv, max_len, D, device=DEV, generator=g).bfloat16() for _ in range(2))
+    kc[:, :, pos + 1:] = float("nan")
+    vc[:, :, pos + 1:] = float("nan")
+    out = torch.empty_like(q)
+    decode_ops.attn_decode(q, kc, vc, torch.tensor([pos], device=DEV), out, nq, D ** -0.5)
+    k, v = (c[:, :, :pos + 1].double().repeat_interleave(nq // nkv, 1) for c in (kc, vc))
+    p = torch.softmax(torch.einsum("bhd,bhtd->bht", q.double().view(B, nq, D), k) * D ** -0.5, -1)
+    ref = torch.einsum("bht,bhtd->bhd", p, v).reshape(B, nq * D)
+    assert rel_l2(out.double().cpu().numpy(), ref.cpu().numpy()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("B,max_len,span", [(30, 4160, 192), (40, 4160, 256), (40, 2500, 128)])
+@pytest.mark.parametrize("spans,rows", [(1, 0), (1, 1), (1, 32), (5, 34), (None, 0)])
+@pytest.mark.parametrize("rising", [False, True])
+def test_attention_spans(B, max_len, span, spans, rows, rising):
+    """A block that walks several times 64 rows: its ring is filled again and again, its last span is short or whole,
+    partial sums are found by the same span; scores that rise with the row, so that every step rescales what is
+    there.  Rows past the position hold NaN."""
+    from helix_substrate_b200 import _lib, decode_ops
+    nq, nkv, D = 8, 4, 64
+    assert _lib.lib().hxq_attn_decode_span(B, nkv, max_len) == span
+    pos = max_len - 1 if spans is None else spans * span + rows - 1
+    g = torch.Generator(device=DEV).manual_seed(pos)
+    q = torch.randn(B, nq * D, device=DEV, generator=g).bfloat16()
+    kc, vc = (torch.randn(B, nkv, max_len, D, device=DEV, generator=g).bfloat16() for _ in range(2))
+    if rising:      # all heads look along the first dimension: scores from 0 to 16, 1 in a step of 260 rows or fewer
+        q.view(B, nq, D)[:, :, 0] = 16.0
+        kc[..., 0] = torch.linspace(0, 8, max_len, device=DEV).bfloat16()
     kc[:, :, pos + 1:] = float("nan")
     vc[:, :, pos + 1:] = float("nan")
     out = torch.empty_like(q)

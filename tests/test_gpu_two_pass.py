@@ -83,6 +83,42 @@ def test_two_passes_against_fp64(M, n_out, n_in, G, xdt, ydt):
     assert _lib.lib().hxq_gemm_scratch_bytes(C.byref(w.desc), M, 1) > 0
 
 
+@pytest.mark.parametrize("M,n_out,n_in,G,tile,rows", [
+    (1030, 64, 2064, 0, 64, 64),            # less than a tile
+    (300, 2573, 272, 0, 96, 2573),          # widths that divide neither the rows nor the accumulator
+    (300, 3566, 272, 0, 128, 3566),
+    (3000, 4619, 1200, 0, 224, 4619),       # three to four tiles per pair of CTAs: both accumulators, used again
+    (2048, 18944, 3584, 128, 256, 9472),    # the widest tile, four per pair, and two runs of rows
+])
+def test_two_passes_tile_widths(M, n_out, n_in, G, tile, rows):
+    """The widths and runs that the rule picks on 148 SMs, with more than one tile per pair where it does."""
+    w, *_ = _check(M, n_out, n_in, G, torch.bfloat16, torch.bfloat16)
+    from helix_substrate_b200 import _lib
+    run = C.c_int32(-1)
+    picked = _lib.lib().hxq_gemm_row_tile(C.byref(w.desc), M, C.byref(run))
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert (picked, run.value) == (tile, rows)
+    assert _lib.lib().hxq_gemm_row_tile(C.byref(w.desc), 128, None) == 0, "one pass"
+
+
+def test_out_of_memory_for_the_scratch_runs_in_one_pass(monkeypatch):
+    """The caching allocator has no room for the bf16 rows: the call runs in one pass on the kept workspace."""
+    from helix_substrate_b200 import _lib
+    w, x, y, ref = _check(1024, 384, 1024, 128, torch.bfloat16, torch.bfloat16)
+    need = _lib.lib().hxq_gemm_scratch_bytes(C.byref(w.desc), 1024, 1)
+    real, refused = torch.empty, []
+
+    def empty(*a, **kw):
+        if kw.get("dtype") == torch.uint8 and a == (need,):
+            refused.append(need)
+            raise torch.OutOfMemoryError("no room")
+        return real(*a, **kw)
+    monkeypatch.setattr(torch, "empty", empty)
+    out = w.matmul(x, torch.bfloat16)
+    assert refused == [need] and w.gemm_status() == 0
+    assert rel_l2(out.double().cpu().numpy(), ref.cpu().numpy()) < TOL
+
+
 def test_two_passes_with_strided_activations_and_no_bias():
     """Rows of x inside a wider matrix: 16-byte aligned (read in place) and not (copied)."""
     for pad in (8, 3):
