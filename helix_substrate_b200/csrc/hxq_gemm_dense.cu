@@ -4,8 +4,8 @@
 //
 //   y[m, o] = sum_k x[m, k] * W[o, k] + bias[o]        (bf16 operands, fp32 accumulator in TMEM)
 //
-// Bound by the staging of its operands (measured below).  A pair of CTAs (one TPC) owns a 256-token x
-// BN-row tile, cta_group::2:
+// Bound by the tensor cores, four fifths of the time, and by the staging of their operands (measured below).  A pair
+// of CTAs (one TPC) owns a 256-token x BN-row tile, cta_group::2:
 //
 //   * the weight rows come blocked, [K / 64][rows][64]: a stage's box is one contiguous piece (as 128-byte
 //     rows 2 K bytes apart a box took several microseconds from HBM, and a product with few token
@@ -22,10 +22,9 @@
 //   * persistent: one pair per TPC walks the tiles in groups of eight token tiles, so that the
 //     tiles running at one time share operands in L2.
 //
-// Measured: 1.46 PFLOP/s on [18944 x 3584] at 2048 and 8192 tokens (0.43 us per 64-column step of a pair's
-// 256 x 256 tile).  It follows the 32 KB that each SM stages per
-// step, 11 TB/s over the GPU, not the MMAs (0.27 us) - a limit of this kernel, not of the machine: the library's
-// product reaches 1.64.
+// Measured: 1.46 PFLOP/s on [18944 x 3584] at 2048 and 8192 tokens.  A 64-column step of a pair's 256 x 256 tile takes
+// 673 cycles (0.43 us at the 1.6 GHz of that load), the tensor pipe being active for 550 of them; in the rest the
+// next stage is waited for, 32 KB per SM and step, 11 TB/s over the GPU.  (The library's product reaches 1.64 PFLOP/s.)
 //
 // BN is a launch argument, a multiple of 32 up to 256 (see pick_tile): an output width that leaves a
 // nearly empty last wave at 256 columns takes the width that fills it.
@@ -314,7 +313,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 // ---- host side ---------------------------------------------------------------------
 
 // Time of a 64-column step of a BN-wide tile, in units of 0.01 us, measured: 0.43 us at 256 columns and 0.33 at
-// 64.  It follows the bytes an SM stages (16 KB of tokens whatever the width), not the MMAs and not the
+// 64.  It follows the bytes an SM stages (16 KB of tokens whatever the width) more than the MMAs, and not the
 // depth of the ring (6 and 11 stages of 64 columns take the same time).
 static int step_cost(int bn) { return 30 + bn / 20; }
 

@@ -64,8 +64,8 @@ void launch_splitk_reduce(const float* partial, int splits, int M, int out_featu
 namespace gemmts {
 
 constexpr int BM = 128;             // output rows per CTA = UMMA M = TMEM lanes
-constexpr int KS = 128;             // K columns per index box (a stage is one or two boxes, see Rings)
-constexpr int DEQ_WARPS = 16;       // four warps per TMEM lane quarter, each takes 32 of a stage's 128 columns
+constexpr int KS = 128;             // K columns per box: one step of the MMAs
+constexpr int DEQ_WARPS = 16;       // four warps per TMEM lane quarter, each takes whole boxes of its own quarter of K
 constexpr int NUM_THREADS = 32 * (2 + DEQ_WARPS);   // activation producer, MMA issuer, 16 dequantisers
 constexpr int LUT_BYTES = 256 * 256;            // entry c, lane l at c * 256 + l * 4, base on a 64 KB boundary
 constexpr int SMEM_TOTAL = 232448;

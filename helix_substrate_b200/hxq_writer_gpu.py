@@ -5,8 +5,8 @@ Follows the reference writer's algorithm (helix_substrate/hxq_writer_v3.py:162-2
 422-467; k-means helix_substrate/hxq_encoder.py:107-207; outliers
 helix_substrate/generate_sidecars_v3.py:18-40) but runs on the GPU, because CPU
 k-means takes about a minute per 16 M-element tensor and a 7B model has 196 of
-them.  On a CUDA device the passes over the weight are kernels (csrc/hxq_encode.cu);
-a CPU tensor takes the same steps in plain torch ops.
+them.  On a CUDA device the passes over the weight are kernels (csrc/hxq_encode.cu), k-means
+on its subsample is plain torch ops; a CPU tensor takes the same steps in torch ops throughout.
 
 Nearest-centroid assignment uses the sorted codebook's midpoints
 (``bucketize``): for a strictly increasing codebook this gives the same index as

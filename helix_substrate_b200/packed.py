@@ -16,7 +16,10 @@ _DT = {torch.float32: HXQ_F32, torch.float16: HXQ_F16, torch.bfloat16: HXQ_BF16}
 
 GEMV_MAX_M = 16      # most tokens hxq_gemv takes per call
 GEMM_TS_MAX_M = 128  # most tokens of the tensor-memory kernel; beyond, hxq_gemm may run in two passes
-GEMV_MAX_M_16BIT = 4  # bf16 / fp16 activations: beyond four tokens the tensor-memory kernel is faster
+# bf16 / fp16 activations: up to four tokens, one launch, hxq_gemv multiplies fp32 weights.  The line is one of precision:
+# the tensor-memory kernel, whose weights are rounded to bf16, takes 28.9 us at five tokens against 38.7 at four on
+# [18944, 3584], and as long on [3584, 18944].  Beyond, every four tokens would read the weights again.
+GEMV_MAX_M_16BIT = 4
 
 
 def uses_gemv(M: int, x_dtype: torch.dtype) -> bool:

@@ -291,8 +291,8 @@ int hxq_allreduce_add_rmsnorm(void* const* peer_buffers, void* const* peer_flags
 
 /*
  * ---- the encoder's passes over a dense fp32 weight (all pointers DEVICE pointers) ----
- * What the reference writer does on the host with numpy (helix_substrate/hxq_encoder.py:107-207,
- * hxq_writer_v3.py:162-232, generate_sidecars_v3.py:18-40), one streaming pass each.
+ * What the reference writer does on the host with numpy (helix_substrate/hxq_writer_v3.py:162-232,
+ * generate_sidecars_v3.py:18-40), one streaming pass each; its k-means is not among them.
  */
 /* out[0], out[1]: the values of 0-based ranks rank0 and rank1 of v[0..n) in ascending order, NaNs last
  * (n < 2^32).  workspace: hxq_encode_select_workspace_bytes() of 8-byte aligned scratch. */
